@@ -786,6 +786,29 @@ def attention_prefill_pooled(q, k_cache, v_cache, block_table, seq_lens, cu_q, m
     return out
 
 
+def _decode_rows_aligned(q) -> bool:
+    return q.data_ptr() % 4 == 0 and q.stride(0) % 2 == 0
+
+
+def _attention_decode(q, k_cache, v_cache, block_table, seq_lens, cu_q, max_q_len, sinks, window, scale, softcap, kv_scales, q_scale, gate, keep_first,
+                      scratch_floats):
+    """Short query segments on the tensor cores (``csrc/cuda/attention_decode.cu``): head dimensions 64 / 128 / 256, bf16 or int8 cache.  The scratch
+    does not depend on the batch and is an ordinary allocation: stream-ordered, and of the graph's own pool under capture."""
+    Tq, n_q, hd = q.shape
+    if kv_scales is not None:
+        assert q_scale is None and gate is None and not keep_first and q.is_contiguous(), "the int8 cache has no gated / position-scaled form"
+    ks, vs = kv_scales if kv_scales is not None else (None, None)
+    scratch = torch.empty(scratch_floats, dtype=torch.float32, device=q.device)
+    out = torch.empty(Tq, n_q, hd, dtype=torch.bfloat16, device=q.device)
+    _check(_lib.cuda().mx_attention_decode(_p(q), _q_rows(q), _p(k_cache), _p(v_cache), _p(ks), _p(vs), _p(block_table), _p(seq_lens), _p(cu_q), _p(sinks),
+                                           _p(gate), 0 if gate is None else gate.stride(0), _p(q_scale), 0 if q_scale is None else q_scale.numel(), _p(out),
+                                           _p(scratch), seq_lens.numel(), Tq, int(max_q_len), n_q, k_cache.shape[1], hd, block_table.shape[1],
+                                           k_cache.shape[2], int(window), int(keep_first), int(gate is not None and gate.shape[1] == n_q), C.c_float(scale),
+                                           C.c_float(softcap), _stream()), "attention_decode")
+    _count()
+    return out
+
+
 def attention(q, k_cache, v_cache, block_table, seq_lens, cu_q, max_q_len, sinks=None, window=0, scale=None, softcap=0.0, n_splits=None,
               kv_scales=None, max_kv_len=0, q_scale=None, gate=None, v_width=0, keep_first=0, pools=None, pool_dense=None, out_rope=None):
     """``v_cache`` None: a value is the first ``v_width`` elements of its key row (latent cache)."""
@@ -809,6 +832,11 @@ def attention(q, k_cache, v_cache, block_table, seq_lens, cu_q, max_q_len, sinks
                                         q_scale=q_scale, gate=gate)
         return attention_prefill_tc(q, k_cache, v_cache, block_table, seq_lens, cu_q, max_q_len, sinks=sinks, window=window, scale=scale,
                                     softcap=softcap, q_scale=q_scale, gate=gate, keep_first=keep_first)
+    if n_splits is None and not extended and v_cache is not None and q.dtype == torch.bfloat16 and hd == dv and _decode_rows_aligned(q):
+        need = _lib.cuda().mx_attention_decode_scratch(hd, B, n_q, n_kv, int(max_q_len))
+        if need:
+            return _attention_decode(q, k_cache, v_cache, block_table, seq_lens, cu_q, max_q_len, sinks, window, scale, softcap, kv_scales, q_scale, gate,
+                                     keep_first, need)
     if n_splits is None:
         # decode-sized problems: split the KV range so that ~2 CTAs per SM exist
         ctas = B * n_kv * max(1, (max_q_len * (n_q // n_kv) + 31) // 32)
