@@ -8,6 +8,7 @@ namespace mx {
 // activation codes: 0 none; 1 SwiGLU, 2 clamped SwiGLU, 3 GeGLU (gated: N columns become N / 2); 4 xIELU, 5 GELU (tanh form),
 // 6 the square of ReLU, 7 tanh (unary)
 constexpr int ACT_CODE_XIELU = 4, ACT_CODE_GELU_TANH = 5, ACT_CODE_RELU2 = 6, ACT_CODE_TANH = 7;
+constexpr int ACT_CODE_SWIGLU = 1, ACT_CODE_SWIGLU_OAI = 2;
 __host__ __device__ constexpr bool act_gated(int act) { return act >= 1 && act <= 3; }
 
 // xIELU: a z^2 + z / 2 for z > 0, b (e^z - 1 - z) + z / 2 otherwise (a = softplus(p), b = 1/2 + softplus(q), formed by the caller).
@@ -101,6 +102,19 @@ template <int V> __device__ __forceinline__ void storev(float* p, const float (&
 template <int V> __device__ __forceinline__ void storev(__nv_bfloat16* p, const float (&v)[V]) {
   if constexpr (V == 4) *reinterpret_cast<uint2*>(p) = make_uint2(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]));
   else *p = __float2bfloat16(v[0]);
+}
+
+// gated pairs of a GEMM epilogue
+__device__ __forceinline__ float glu_apply(int act, float g, float u, float alpha, float limit) {
+  if (act == ACT_CODE_SWIGLU) return g / (1.f + __expf(-g)) * u;
+  if (act == ACT_CODE_SWIGLU_OAI) {
+    g = fminf(g, limit);
+    u = fminf(fmaxf(u, -limit), limit);
+    return g / (1.f + __expf(-alpha * g)) * (u + 1.f);
+  }
+  // GeGLU, tanh approximation
+  const float t = tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g));
+  return 0.5f * g * (1.f + t) * u;
 }
 
 }  // namespace mx

@@ -28,7 +28,7 @@ constexpr int BK = 64;
 constexpr int kNumEpilogueWarps = 4;
 constexpr int kNumDequantWarps = 8;
 
-enum Act : int { ACT_NONE = 0, ACT_SWIGLU = 1, ACT_SWIGLU_OAI = 2, ACT_GEGLU = 3 };      // unary codes: act.cuh
+constexpr int ACT_NONE = 0;                      // codes: act.cuh
 
 struct GemmParams {
   int M, N, K;
@@ -100,18 +100,6 @@ __device__ __forceinline__ void tile_coords(int t, int m_tiles, int n_tiles, int
   mt = g * group_m + r % gm;
   nt = r / gm;
   if (m_rot) { mt += m_rot; if (mt >= m_tiles) mt -= m_tiles; }
-}
-
-__device__ __forceinline__ float act_apply(int act, float g, float u, float alpha, float limit) {
-  if (act == ACT_SWIGLU) return g / (1.f + __expf(-g)) * u;
-  if (act == ACT_SWIGLU_OAI) {
-    g = fminf(g, limit);
-    u = fminf(fmaxf(u, -limit), limit);
-    return g / (1.f + __expf(-alpha * g)) * (u + 1.f);
-  }
-  // GeGLU, tanh approximation
-  const float t = tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g));
-  return 0.5f * g * (1.f + t) * u;
 }
 
 template <int FMT, int BN, int SA, int SB>
@@ -382,7 +370,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
           const int ocol0 = col0 >> 1;
           float o[16];
 #pragma unroll
-          for (int j = 0; j < 16; ++j) o[j] = act_apply(p.act, v[j], v[16 + j], p.act_alpha, p.act_limit) * rs;
+          for (int j = 0; j < 16; ++j) o[j] = glu_apply(p.act, v[j], v[16 + j], p.act_alpha, p.act_limit) * rs;
           const int on = p.N >> 1;
           if (p.out_f32 == 1) {
             float* out = (float*)p.C + (size_t)row * p.ldc + ocol0;

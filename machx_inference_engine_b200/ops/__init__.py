@@ -71,8 +71,16 @@ def _make(name):
     return op
 
 
+def expert_chunk(w, rows_per_expert):
+    """See :func:`ops.cuda.expert_chunk`; the oracle's grouped product ignores it."""
+    if not w.p0.is_cuda:
+        return 0
+    from . import cuda
+    return cuda.expert_chunk(w, rows_per_expert)
+
+
 for _n in _NAMES:
     globals()[_n] = _make(_n)
 
-__all__ = _NAMES + ["set_backend", "QuantWeight", "WFormat", "from_dense", "from_exl3", "from_ggml", "BranchMean", "ExpertSum", "MoePacking", "PoolPages", "moe_max_rows", "ACT_NONE", "ACT_SWIGLU",
+__all__ = _NAMES + ["set_backend", "expert_chunk", "QuantWeight", "WFormat", "from_dense", "from_exl3", "from_ggml", "BranchMean", "ExpertSum", "MoePacking", "PoolPages", "moe_max_rows", "ACT_NONE", "ACT_SWIGLU",
                     "ACT_SWIGLU_OAI", "ACT_GEGLU", "ACT_XIELU", "ACT_GELU_TANH", "ACT_RELU2", "ACT_TANH", "act_gated", "MOE_TILE"]

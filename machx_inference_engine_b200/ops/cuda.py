@@ -527,6 +527,49 @@ def _few_rows_take_gemm(M: int, w: QuantWeight, act: int) -> bool:
     return (M >= 3 and 2 * M * w.K + 16 * min(w.K, 4096) > 190 * 1024) or (M >= 5 and w.N * w.K >= 48 << 20)
 
 
+GEMM_ROWS_MAX = 64        # activation rows per group of the weight-streaming kernel (csrc/cuda/gemm_rows.cu)
+
+
+def _takes_rows(x, w: QuantWeight, act: int, row_scale) -> bool:
+    """Whether a dense layer of a few rows takes the weight-streaming kernel.  Measured with cold caches (us, GEMV or tcgen05 kernel -> this one):
+    two rows stay with the GEMV (6144 x 4096: bf16 21.4 -> 22.6, Q8 19.3 -> 23.5) except for gated bf16 and Q8 (28672 x 4096: 104 -> 58, 56 -> 42), which it reads
+    once per row; three rows 27.5 -> 23.4 and 25.4 -> 23.4, eight 55 -> 23 and 48 -> 24, forty 38 -> 29 and 64 -> 36.  Above: bf16 48 rows 38 -> 30, 64 rows
+    38 -> 34 but 30 -> 33 for 5120 x 2880; matrices of several full waves (from 100 M elements) are already near the memory rate in the tcgen05
+    kernel: 28672 x 4096 33 rows 71 -> 63, 48 rows 71 -> 70, 32768 x 4096 24 rows 68 -> 66, 33 rows 68.6 -> 69.7.  Q8 48 rows 64 -> 32 and 97 -> 76, 64 rows
+    54 -> 47 and 142 -> 106 (there the other kernels decode the weight once), 56 rows of 32768 x 4096 97 -> 104."""
+    M, big = x.shape[0], w.N * w.K >= 100 << 20
+    if w.fmt == WFormat.BF16:
+        most = 32 if big else 48
+    elif w.fmt == WFormat.Q8:
+        most = 48 if big else GEMM_ROWS_MAX
+    else:
+        return False
+    least = 2 if act_gated(act) else 3
+    if row_scale is not None:
+        least = 1                        # (the GEMVs have no row scale)
+    return least <= M <= most and w.K % 8 == 0 and x.data_ptr() % 16 == 0 and w.p0.data_ptr() % 16 == 0
+
+
+def expert_chunk(w: QuantWeight, rows_per_expert: float) -> int:
+    """Rows per group with which a bank of experts takes the weight-streaming kernel, 0: the grouped tcgen05 kernel.  Q8 banks, gate / up and down, us at the mean
+    rows per expert (tcgen05 -> this kernel, groups of 8 / 16): 512 experts of 1024 x 2048: 0.6 rows 499 -> 206 / 210, 2.5 rows 957 -> 376 / 382,
+    10 rows 1082 -> 753 / 603, 19.5 rows 1174 -> 1248 / 888, 29 rows 1164 -> 1173; 128 of 1536 x 2048: 16 rows 433 -> 300, 32 rows 413 -> 468."""
+    if w.fmt != WFormat.Q8 or rows_per_expert > 24:
+        return 0
+    return 8 if rows_per_expert <= 3 else 16
+
+
+def _gemm_rows(x, w: QuantWeight, out, out_kind, bias, row_scale, act, act_alpha, act_limit, chunk, tiles=None):
+    """``tiles``: (tile_expert, tile_valid, num_tiles) of packed expert rows, taken in groups of ``chunk``.  The scratch (partials of cut tiles) is an ordinary
+    allocation: stream-ordered, of the graph's own pool under capture."""
+    lib = _lib.cuda()
+    scratch = torch.empty(lib.mx_gemm_rows_scratch(chunk), dtype=torch.float32, device=x.device)
+    te, tv, nt = tiles if tiles is not None else (None, None, None)
+    _check(lib.mx_gemm_rows(_p(x), int(w.fmt), _p(w.p0), _p(w.p1), w.E, _p(out), out.stride(0), out_kind, _p(bias), _p(row_scale), act, C.c_float(act_alpha),
+                            C.c_float(act_limit), x.shape[0], w.N, w.K, _p(te), _p(tv), _p(nt), 0 if te is None else te.numel(), int(chunk), _p(scratch),
+                            _stream()), "gemm_rows")
+
+
 def linear(x, w: QuantWeight, bias=None, act=ACT_NONE, act_alpha=1.702, act_limit=7.0, out_f32=False, row_scale=None, out=None):
     """``out``: write into this [M, n_out] view (unit column stride; a column slice of a wider matrix is fine), so that projections
     whose weights differ in format can share one output without a concatenation."""
@@ -546,7 +589,9 @@ def linear(x, w: QuantWeight, bias=None, act=ACT_NONE, act_alpha=1.702, act_limi
         return out
     fmt, p0, p1, p2, p3 = _planes(w)
     lib = _lib.cuda()
-    if M <= GEMV_MAX_M and row_scale is None and not _few_rows_take_gemm(M, w, act):
+    if _takes_rows(x, w, act, row_scale):
+        _gemm_rows(x, w, out, _out_kind(odt), bias, row_scale, act, act_alpha, act_limit, M)
+    elif M <= GEMV_MAX_M and row_scale is None and not _few_rows_take_gemm(M, w, act):
         # the GEMV kernels write dense rows: a strided view of more than one row goes through a dense buffer
         dst = out if (M == 1 or out.stride(0) == n_out) else torch.empty(M, n_out, dtype=odt, device=x.device)
         _check(lib.mx_gemv(fmt, p0, p1, p2, p3, _p(x), _p(dst), _p(bias), M, w.N, w.K, int(out_f32), act, C.c_float(act_alpha),
@@ -660,8 +705,9 @@ def gemm(x, w: QuantWeight, bias=None, act=ACT_NONE, act_alpha=1.702, act_limit=
 
 
 def grouped_linear(xp, w: QuantWeight, tile_expert, num_tiles, bias=None, act=ACT_NONE, act_alpha=1.702, act_limit=7.0, out_f32=False, bn=128,
-                   out_dtype=None):
-    """``out_dtype`` (bf16 / fp16 / fp32) overrides ``out_f32``; fp16 feeds a following MXFP4 GEMM without a cast."""
+                   out_dtype=None, tile_valid=None, chunk=0):
+    """``chunk`` > 0 (with ``tile_valid``, the live rows of every tile): the weight-streaming kernel over groups of that many rows, for experts of a few dozen
+    rows each; rows past a tile's live ones are then not written.  ``out_dtype`` (bf16 / fp16 / fp32) overrides ``out_f32``; fp16 feeds a following MXFP4 GEMM without a cast."""
     P = xp.shape[0]
     if xp.dtype == torch.float32:            # 32-bit models: every row in fp32 on the CUDA cores
         if w.fmt != WFormat.BF16 or bias is not None or out_dtype not in (None, torch.float32):
@@ -678,6 +724,10 @@ def grouped_linear(xp, w: QuantWeight, tile_expert, num_tiles, bias=None, act=AC
     out = torch.empty(P, n_out, dtype=odt, device=xp.device)
     fmt, p0, p1, p2, p3 = _planes(w)
     xp = _gemm_a(xp, w)
+    if chunk and tile_valid is not None and w.fmt in (WFormat.BF16, WFormat.Q8) and tile_expert.numel() <= 1024:
+        _gemm_rows(xp, w, out, _out_kind(odt), bias, None, act, act_alpha, act_limit, chunk, tiles=(tile_expert, tile_valid, num_tiles))
+        _count()
+        return out
     _check(_lib.cuda().mx_gemm(_p(xp), fmt, p0, p1, p2, p3, w.E, _p(out), n_out, _out_kind(odt), _p(bias), _vp(0), act, C.c_float(act_alpha),
                                C.c_float(act_limit), P, w.N, w.K, _p(tile_expert), _p(num_tiles), bn, _stream()), "grouped gemm")
     _count()
