@@ -63,10 +63,10 @@ template <> struct FaArgs<2> { using T = FaPoolParams; };
 
 template <int DK, int DV>
 struct FaCfg {
-  static constexpr int BKV = (DK <= 128 && DV <= 128) ? 128 : 64;   // keys per tile
+  static constexpr int BKV = 64;                               // keys per tile
   static constexpr int NS = 2;                                 // S buffers in TMEM
-  static constexpr int CTAS = 1;                               // one CTA per SM: its softmax threads keep a whole S row in registers
-  static constexpr uint32_t TMEM_COLS = 512;
+  static constexpr int CTAS = (DK <= 128 && DV <= 128) ? 2 : 1;
+  static constexpr uint32_t TMEM_COLS = 512 / CTAS;
   static constexpr int KATOMS = DK / 64, VATOMS = DV / 64;     // 64-column (128-byte) swizzle atoms per row of Q / K and of V
   static constexpr int Q_BYTES = FA_BQ * DK * 2;
   static constexpr int K_BYTES = BKV * DK * 2, V_BYTES = BKV * DV * 2;
@@ -77,7 +77,7 @@ struct FaCfg {
   static constexpr int V_OFF = K_OFF + KS * K_BYTES;
   static constexpr int P_OFF = V_OFF + VS * V_BYTES;
   static constexpr int BAR_OFF = P_OFF + P_BYTES;
-  static constexpr int TOTAL = BAR_OFF + 256 + 1024;
+  static constexpr int TOTAL = BAR_OFF + 256 + (CTAS == 2 ? 512 : 1024);
   static_assert(TOTAL <= 232448, "shared memory plan exceeds 227 KB");
   static_assert(NS * BKV + DV <= (int)TMEM_COLS, "TMEM plan");
 };

@@ -1,7 +1,7 @@
 """Weight-streaming products of a few rows (csrc/cuda/gemm_rows.cu) against fp64.
 
 Bound: the operands are exact (bf16, or int8 codes and fp16 scales), the sums fp32.  Rounding to bf16 moves an element, and so the 2-norm, by at most
-2^-9 = 1.95e-3; fp32 results differ by the order of the sums, about 1e-6, and by what the tensor cores cut off:
+2^-8 = 3.9e-3; fp32 results differ by the order of the sums, about 1e-6, and by what the tensor cores cut off:
 up to a unit in the last place of the running sum (2^-23) at each of the K / 16 additions, half of it on average."""
 import pytest
 import torch
@@ -49,7 +49,7 @@ def test_rows_and_ragged_weights(fmt, M, N, Kd):
     tol = 3e-6 + Kd / 16 * 2.0 ** -24
     assert rel(product(x, w, True), want) < tol
     got = product(x, w, False)
-    assert rel(got, want) < 2e-3
+    assert rel(got, want) < 2.0 ** -8
     assert torch.equal(got, product(x, w, False))                    # the parts of a cut tile are added in a fixed order
     bias, rs = torch.randn(N, device=x.device), torch.rand(M, device=x.device)
     assert rel(product(x, w, True, bias=bias, row_scale=rs), (want + bias.double()) * rs.double()[:, None]) < tol
@@ -65,7 +65,7 @@ def test_activations(fmt, act):
     assert rel(got.cpu(), want) < 5e-3                               # (the oracle's Q8 weights are rounded to bf16)
     wide = torch.zeros(19, got.shape[1] + 24, dtype=torch.bfloat16, device="cuda:0")
     ops.linear(x, w, act=act, out=wide[:, 8:8 + got.shape[1]])
-    assert rel(wide[:, 8:8 + got.shape[1]], got) < 2e-3 and float(wide[:, :8].abs().max()) == 0 and float(wide[:, 8 + got.shape[1]:].abs().max()) == 0
+    assert rel(wide[:, 8:8 + got.shape[1]], got) < 2.0 ** -8 and float(wide[:, :8].abs().max()) == 0 and float(wide[:, 8 + got.shape[1]:].abs().max()) == 0
 
 
 @pytest.mark.parametrize("fmt", [WFormat.BF16, WFormat.Q8])
