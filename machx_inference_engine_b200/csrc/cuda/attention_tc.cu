@@ -11,16 +11,21 @@
 // [128] that pool_blocks (pooled.cu) has written for the step, as tiles in front of the window's.  This mode also takes the soft-cap as a parameter, through
 // an accurate tanh, and may turn the output back by the query's position (a rotation of neighbouring pairs, before the gate).
 //
-// One CTA owns 128 query tokens of one query head and walks the key tiles of its range (128 keys per tile, 64 for
-// head_dim 256 so that two K and two V tiles still fit in shared memory):
+// One CTA owns 128 query tokens of one query head and walks the key tiles of its range, 64 keys per tile; with heads of up to 128 columns two CTAs share
+// an SM (256 TMEM columns each):
 //   warp 0  : TMA loads of the K and V tiles (two-stage rings) and, once, of the Q tile
 //   warp 1  : tcgen05.mma  S(j) = Q K_j^T  into one of two S buffers in TMEM, so that S(j+1) is computed while the softmax
-//             threads work on S(j);  O += P_j V_j  accumulates in TMEM over all tiles
-//   warps 2-5 (one thread per query row = TMEM lane): read S, mask, online softmax, write P (bf16) into a 128-byte-swizzled
-//             shared tile for the PV MMA.  The output row is NOT kept in registers: O stays in TMEM and is rescaled in place
+//             threads work on S(j);  O += P_j V_j  accumulates in TMEM over all tiles, with P_j as its A operand in TMEM
+//   warps 2-5 (one thread per query row = TMEM lane): read S, mask, online softmax, write P (bf16) over the S they have read.
+//             The output row is NOT kept in registers: O stays in TMEM and is rescaled in place
 //             (tcgen05.ld / tcgen05.st) only when the running maximum has grown by more than 2^8 since the last rescale;
 //             until then P is formed against the old reference maximum (it stays far inside bf16's range) and O and the
 //             denominator remain consistent.  That removes the per-tile fold of O and is what lets head_dim 256 fit.
+//
+// Bound: the exponentials (16 per SM and cycle: 122 us for 4096 causal tokens of 64 heads, against 85 us of tensor time with heads of 64).  One softmax
+// warp per scheduler cannot hide its own chain of TMEM read, maximum, exponentials and write, hence two CTAs per SM with half the tile each, P that never
+// passes shared memory, and packed fp32 arithmetic.
+// MEASURED
 // The per-head sink joins the denominator once, at the end.  Every wait is bounded.
 //
 // Reference parity: src/ops/attention.cpp:2456-2815 (fa2_tile_wide_impl<HD,Bc,REGDOT,SG,SINK> for HD 64..512 and its
@@ -71,13 +76,11 @@ struct FaCfg {
   static constexpr int Q_BYTES = FA_BQ * DK * 2;
   static constexpr int K_BYTES = BKV * DK * 2, V_BYTES = BKV * DV * 2;
   static constexpr int KS = 2, VS = 2;                         // tiles in flight
-  static constexpr int P_BYTES = FA_BQ * BKV * 2;
   static constexpr int Q_OFF = 0;
   static constexpr int K_OFF = Q_OFF + Q_BYTES;
   static constexpr int V_OFF = K_OFF + KS * K_BYTES;
-  static constexpr int P_OFF = V_OFF + VS * V_BYTES;
-  static constexpr int BAR_OFF = P_OFF + P_BYTES;
-  static constexpr int TOTAL = BAR_OFF + 256 + (CTAS == 2 ? 512 : 1024);
+  static constexpr int BAR_OFF = V_OFF + VS * V_BYTES;
+  static constexpr int TOTAL = BAR_OFF + 256 + 1024;
   static_assert(TOTAL <= 232448, "shared memory plan exceeds 227 KB");
   static_assert(NS * BKV + DV <= (int)TMEM_COLS, "TMEM plan");
 };
@@ -121,6 +124,22 @@ __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
   uint64_t d;
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
+}
+
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+
+// D[tmem] (+)= A[tmem] * B[smem]: A is bf16, a row per lane, two elements per 32-bit column
+__device__ __forceinline__ void umma_bf16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
 }
 
 // v x P(v^2) over a run, P of degree D with the coefficients c (of rising powers)
@@ -180,19 +199,20 @@ fa_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
   constexpr int BKV = L::BKV, NS = L::NS, KS = L::KS, VS = L::VS;
   constexpr float LOG2E = 1.4426950408889634f;
   constexpr float RESCALE_STEP = 8.f;            // in log2 units: O is rescaled when the maximum has grown by a factor of 256
-  extern __shared__ uint8_t smem_raw[];
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   const uint32_t sbase = smem_u32(smem);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::BAR_OFF);
-  // barriers: q_full, k_full[2], v_full[2], k_empty[2], v_empty[2], s_full[2], s_empty[2], p_full, pv_done
+  // barriers: q_full, k_full[2], v_full[2], k_empty[2], v_empty[2], s_full[2], p_full[2], pv_done[2]
   const uint32_t b_qfull = smem_u32(bars), b_kfull = b_qfull + 8, b_vfull = b_kfull + 16, b_kempty = b_vfull + 16, b_vempty = b_kempty + 16;
-  const uint32_t b_sfull = b_vempty + 16, b_sempty = b_sfull + 16, b_pfull = b_sempty + 16, b_pvdone = b_pfull + 8;
+  const uint32_t b_sfull = b_vempty + 16, b_pfull = b_sfull + 16, b_pvdone = b_pfull + 16;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int b = blockIdx.x / p.max_q_tiles, qt = blockIdx.x % p.max_q_tiles;
-  const int head = blockIdx.y;
+  // CTAs start in the order of the last query tiles first (causal: those with the most keys), over all heads and sequences: the short ones fill the end
+  const int head = blockIdx.x % p.n_q, rest = blockIdx.x / p.n_q, n_seqs = gridDim.x / p.n_q / p.max_q_tiles;
+  const int b = rest % n_seqs, qt = p.max_q_tiles - 1 - rest / n_seqs;
   const int kvh = head / (p.n_q / p.n_kv);
   const int q_begin = p.cu_q[b], q_len = p.cu_q[b + 1] - q_begin;
   const int t0 = qt * FA_BQ;
@@ -225,9 +245,8 @@ fa_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
     mbar_init(b_qfull, 1);
     for (int s = 0; s < 2; ++s) {
       mbar_init(b_kfull + 8 * s, 1); mbar_init(b_vfull + 8 * s, 1); mbar_init(b_kempty + 8 * s, 1); mbar_init(b_vempty + 8 * s, 1);
-      mbar_init(b_sfull + 8 * s, 1); mbar_init(b_sempty + 8 * s, 4);
+      mbar_init(b_sfull + 8 * s, 1); mbar_init(b_pfull + 8 * s, 4); mbar_init(b_pvdone + 8 * s, 1);
     }
-    mbar_init(b_pfull, 4); mbar_init(b_pvdone, 1);
     *abort_flag = 0;
     fence_mbar_init();
   }
@@ -278,11 +297,12 @@ fa_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       constexpr uint32_t idesc_s = umma_idesc_bf16(FA_BQ, BKV, 0, 0);
       constexpr uint32_t idesc_o = umma_idesc_bf16(FA_BQ, DV, 0, 1);      // B = V is MN-major (head_dim contiguous)
       bool ok = mbar_wait(b_qfull, 0, p.status, ERR_MBAR_TIMEOUT_MMA, abort_flag);
-      // S(j) = Q K_j^T into S buffer j % NS (waits for K_j and for the softmax threads to have released that buffer)
+      // Phases: a barrier per S buffer, of tiles j, j + NS, ..  S(j) is issued after PV(j - NS) has completed, so whoever works on tile j finds the barriers of
+      // tiles j and j - 1 at most one phase behind: one parity bit tells the two apart.
+      // S(j) = Q K_j^T into S buffer j % NS, whose tile j - NS has been multiplied (P(j - NS) lies in it)
       auto issue_s = [&](int j) -> bool {
-        const uint32_t sk = j % KS, phk = (j / KS) & 1, sb = j % NS, phs = (j / NS) & 1;
+        const uint32_t sk = j % KS, phk = (j / KS) & 1, sb = j % NS;
         if (!mbar_wait(b_kfull + 8 * sk, phk, p.status, ERR_MBAR_TIMEOUT_MMA, abort_flag)) return false;
-        if (!mbar_wait(b_sempty + 8 * sb, phs ^ 1, p.status, ERR_MBAR_TIMEOUT_MMA, abort_flag)) return false;
         tc_fence_after();
         const uint32_t qa = sbase + L::Q_OFF, ka = sbase + L::K_OFF + sk * L::K_BYTES;
 #pragma unroll
@@ -295,23 +315,20 @@ fa_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         umma_commit(b_kempty + 8 * sk);
         return true;
       };
-      if (ok && n_tiles > 0) ok = issue_s(0);
+      for (int j = 0; j < min(NS, n_tiles) && ok; ++j) ok = issue_s(j);
       for (int j = 0; j < n_tiles && ok; ++j) {
-        if (NS == 2 && j + 1 < n_tiles && !(ok = issue_s(j + 1))) break;       // the next score tile runs while softmax(j) works
         const uint32_t sv = j % VS, phv = (j / VS) & 1;
-        if (!(ok = mbar_wait(b_pfull, j & 1, p.status, ERR_MBAR_TIMEOUT_MMA, abort_flag))) break;
         if (!(ok = mbar_wait(b_vfull + 8 * sv, phv, p.status, ERR_MBAR_TIMEOUT_MMA, abort_flag))) break;
+        if (!(ok = mbar_wait(b_pfull + 8 * (j % NS), (j / NS) & 1, p.status, ERR_MBAR_TIMEOUT_MMA, abort_flag))) break;
         tc_fence_after();
-        const uint32_t pa = sbase + L::P_OFF, va = sbase + L::V_OFF + sv * L::V_BYTES;
+        const uint32_t pa = tmem_base + (j % NS) * BKV, va = sbase + L::V_OFF + sv * L::V_BYTES;
 #pragma unroll
-        for (int kk = 0; kk < BKV / 16; ++kk) {
-          const uint64_t ad = umma_desc_k_sw128(pa + (kk >> 2) * (FA_BQ * 128) + (kk & 3) * 32);
-          const uint64_t bd = umma_desc_mn_sw128(va + kk * 2048, BKV * 128, 1024);
-          umma_bf16(tmem_o, ad, bd, idesc_o, (j | kk) != 0);
-        }
-        umma_commit(b_pvdone);
+        for (int kk = 0; kk < BKV / 16; ++kk)          // 16 keys of P: eight TMEM columns
+          umma_bf16_ts(tmem_o, pa + kk * 8, umma_desc_mn_sw128(va + kk * 2048, BKV * 128, 1024), idesc_o, (j | kk) != 0);
+        umma_commit(b_pvdone + 8 * (j % NS));
         umma_commit(b_vempty + 8 * sv);
-        if (NS == 1 && j + 1 < n_tiles && !(ok = issue_s(j + 1))) break;
+        // the next score tile of this buffer overwrites P(j); meanwhile the softmax threads work on the other buffer
+        if (j + NS < n_tiles && (!(ok = mbar_wait(b_pvdone + 8 * (j % NS), (j / NS) & 1, p.status, ERR_MBAR_TIMEOUT_MMA, abort_flag)) || !(ok = issue_s(j + NS)))) break;
       }
     }
   } else {
@@ -350,9 +367,6 @@ fa_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
 #pragma unroll
       for (int cb = 0; cb < BKV; cb += 32) tmem_ld_32x32(ts + cb, *reinterpret_cast<uint32_t(*)[32]>(&sv[cb]));
       tmem_ld_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(b_sempty + 8 * sb);
       const int key0 = first_key(j);
       bool capped = false;
       if constexpr (MODE == 2) {
@@ -394,12 +408,10 @@ fa_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
           }
         }
       }
-      float tmax = sv[0];
+      float mx[4] = {sv[0], sv[1], sv[2], sv[3]};      // four chains: one alone would be 64 dependent instructions
 #pragma unroll
-      for (int i = 1; i < BKV; ++i) tmax = fmaxf(tmax, sv[i]);
-      tmax *= c;                                   // c > 0
-      // P(j) overwrites the shared tile PV(j-1) reads, and a rescale touches the accumulator PV(j-1) writes: both wait for it
-      if (j > 0 && !(ok = mbar_wait(b_pvdone, (j - 1) & 1, p.status, ERR_MBAR_TIMEOUT_SOFTMAX, abort_flag))) break;
+      for (int i = 4; i < BKV; ++i) mx[i & 3] = fmaxf(mx[i & 3], sv[i]);
+      const float tmax = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * c;      // c > 0
       // tcgen05.ld / tcgen05.st are warp-wide instructions: the decision to rescale is taken per warp, and a row whose own
       // maximum has not grown simply rescales by 1
       const bool grow = tmax > m + RESCALE_STEP || j == 0;
@@ -407,6 +419,7 @@ fa_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       if (j > 0 && __any_sync(0xffffffffu, grow)) {
         const float alpha = ex2_fast(m - m_new);
         l *= alpha;
+        if (!(ok = mbar_wait(b_pvdone + 8 * ((j - 1) % NS), ((j - 1) / NS) & 1, p.status, ERR_MBAR_TIMEOUT_SOFTMAX, abort_flag))) break;      // PV(j-1) writes the accumulator
         tc_fence_after();
 #pragma unroll 1
         for (int cb = 0; cb < DV; cb += 32) {
@@ -420,29 +433,30 @@ fa_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
         tmem_st_wait();
       }
       m = m_new;
-      float psum = 0.f;
-      const float neg_m = -m;
+      const uint64_t c2 = pack2(c, c), neg_m2 = pack2(-m, -m);
+      uint64_t psum[2] = {0ull, 0ull};
 #pragma unroll
-      for (int cb = 0; cb < BKV; cb += 32) {
-        uint32_t pk[16];
+      for (int cb = 0; cb < BKV; cb += 64) {
+        uint32_t pk[32];
 #pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          const float p0 = ex2_fast(fmaf(sv[cb + i], c, neg_m)), p1 = ex2_fast(fmaf(sv[cb + i + 1], c, neg_m));
-          psum += p0 + p1;
+        for (int i = 0; i < 64; i += 2) {
+          float p0, p1;
+          unpack2(fma2(pack2(sv[cb + i], sv[cb + i + 1]), c2, neg_m2), p0, p1);
+          p0 = ex2_fast(p0);
+          p1 = ex2_fast(p1);
+          psum[(i >> 1) & 1] = add2(psum[(i >> 1) & 1], pack2(p0, p1));
           pk[i >> 1] = pack_bf16(p0, p1);
         }
-        // 32 keys = 64 bytes = 4 chunks of this row, in atom (cb / 64), chunks (cb % 64) / 8 ..
-        uint8_t* prow = smem + L::P_OFF + (cb >> 6) * (FA_BQ * 128);
-        const int ch0 = (cb & 63) >> 3;
-#pragma unroll
-        for (int ch = 0; ch < 4; ++ch)
-          *reinterpret_cast<uint4*>(prow + sw128_offset(r, ch0 + ch)) = make_uint4(pk[4 * ch], pk[4 * ch + 1], pk[4 * ch + 2], pk[4 * ch + 3]);
+        tmem_st_32x32(ts + (cb >> 1), pk);           // P(j) over S(j): two keys per column
       }
-      l += psum;
-      tc_fence_before();            // a rescale's TMEM stores, before the MMA thread is told to accumulate into O again
-      fence_proxy_async();          // the P tile, written through the generic proxy, before the MMA reads it
+      float s0, s1, s2, s3;
+      unpack2(psum[0], s0, s1);
+      unpack2(psum[1], s2, s3);
+      l += (s0 + s1) + (s2 + s3);
+      tmem_st_wait();
+      tc_fence_before();            // P and a rescale's stores, before the MMA thread is told to multiply
       __syncwarp();
-      if (lane == 0) mbar_arrive(b_pfull);
+      if (lane == 0) mbar_arrive(b_pfull + 8 * sb);
     }
     const int dv = p.dv;
     const __nv_bfloat16* grow = p.gate && !p.gate_heads && row_ok ? p.gate + (size_t)(q_begin + t0 + r) * p.gate_ld + (size_t)head * dv : nullptr;
@@ -454,7 +468,7 @@ fa_prefill_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_const
       for (int i = 0; i < GPRE / 8; ++i)
         if (8 * i < dv) gpre[i] = __ldg(reinterpret_cast<const uint4*>(grow + 8 * i));
     }
-    if (ok && n_tiles > 0) ok = mbar_wait(b_pvdone, (n_tiles - 1) & 1, p.status, ERR_MBAR_TIMEOUT_SOFTMAX, abort_flag);
+    if (ok && n_tiles > 0) ok = mbar_wait(b_pvdone + 8 * ((n_tiles - 1) % NS), ((n_tiles - 1) / NS) & 1, p.status, ERR_MBAR_TIMEOUT_SOFTMAX, abort_flag);
     if (ok) {
       tc_fence_after();
       if (p.sinks) l += ex2_fast(p.sinks[head] * LOG2E - m);
@@ -554,7 +568,7 @@ static int launch_fa(const void* q, const void* k_cache, const void* v_cache, co
     if (e != cudaSuccess) return (int)e;
     configured.mark();
   }
-  dim3 grid(B * p.max_q_tiles, p.n_q);
+  dim3 grid(p.n_q * B * p.max_q_tiles);
   kern<<<grid, 192, L::TOTAL, st>>>(tq, tk, tv, tq, tk, p);
   return (int)cudaGetLastError();
 }
@@ -595,7 +609,7 @@ static int launch_fa_split(const void* q, const FaSplit& x, const FaParams& p, i
     if (e != cudaSuccess) return (int)e;
     configured.mark();
   }
-  kern<<<dim3(B * p.max_q_tiles, p.n_q), 192, L::TOTAL, st>>>(tq, tk, tv, tqr, tkr, p);
+  kern<<<dim3(p.n_q * B * p.max_q_tiles), 192, L::TOTAL, st>>>(tq, tk, tv, tqr, tkr, p);
   return (int)cudaGetLastError();
 }
 
@@ -627,7 +641,7 @@ static int launch_fa_pooled(const void* q, const void* k_cache, const void* v_ca
     if (e != cudaSuccess) return (int)e;
     configured.mark();
   }
-  kern<<<dim3(B * p.max_q_tiles, p.n_q), 192, L::TOTAL, st>>>(tq, tk, tv, tpk, tpv, p);
+  kern<<<dim3(p.n_q * B * p.max_q_tiles), 192, L::TOTAL, st>>>(tq, tk, tv, tpk, tpv, p);
   return (int)cudaGetLastError();
 }
 
