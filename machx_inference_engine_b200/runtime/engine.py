@@ -19,6 +19,7 @@ from collections import OrderedDict, deque
 from dataclasses import dataclass, field
 from typing import Callable, Iterable, Optional
 
+import numpy as np
 import torch
 
 from .. import ops
@@ -469,46 +470,63 @@ class LLMEngine:
     def _build_batch(self, plan: list, logit_rows: list, pad_to: int = 0):
         """``logit_rows``: rows of the flattened batch whose logits are computed."""
         logit_rows = list(logit_rows)
-        ids, pos, slots, cu, lens, tables = [], [], [], [0], [], []
+        B, mb = len(plan), self.max_blocks_per_seq
+        pad = max(0, pad_to - B)                           # graph padding: null sequences of one token in block 0
+        T = sum(n for _, n in plan) + pad
+        ids, pos, slots = np.zeros(T, np.int32), np.zeros(T, np.int32), np.full(T, -1, np.int64)
+        cu, lens, bt = np.zeros(B + pad + 1, np.int32), np.ones(B + pad, np.int32), np.zeros((B + pad, mb), np.int32)
+        at = 0
         for i, (seq, n) in enumerate(plan):
             s0 = seq.n_computed
-            ids.extend(seq.tokens[s0:s0 + n])
-            pos.extend(range(s0, s0 + n))
-            for p_ in range(s0, s0 + n):
-                slots.append(seq.blocks[p_ // KV_BLOCK] * KV_BLOCK + p_ % KV_BLOCK)
-            cu.append(cu[-1] + n)
-            lens.append(s0 + n)
-            tables.append(seq.blocks)
-        B = len(plan)
-        for _ in range(max(0, pad_to - B)):                # graph padding: null sequences of one token in block 0
-            ids.append(0); pos.append(0); slots.append(-1); cu.append(cu[-1] + 1); lens.append(1); tables.append([0])
-            logit_rows.append(cu[-1] - 1)
-        mb = self.max_blocks_per_seq
-        bt = torch.zeros(len(tables), mb, dtype=torch.int32)
-        for r, t in enumerate(tables):
-            if len(t) > mb:
+            if len(seq.blocks) > mb:
                 raise ContextLengthExceeded("sequence outgrew the block table")
-            bt[r, :len(t)] = torch.tensor(t, dtype=torch.int32)
-        extra = {}
+            bt[i, :len(seq.blocks)] = seq.blocks
+            if n == 1:
+                ids[at], pos[at], slots[at] = seq.tokens[s0], s0, seq.blocks[s0 // KV_BLOCK] * KV_BLOCK + s0 % KV_BLOCK
+            else:
+                ids[at:at + n] = seq.tokens[s0:s0 + n]
+                p = np.arange(s0, s0 + n)
+                pos[at:at + n] = p
+                slots[at:at + n] = bt[i, p // KV_BLOCK].astype(np.int64) * KV_BLOCK + p % KV_BLOCK
+            at += n
+            cu[i + 1], lens[i] = at, s0 + n
+        for i in range(pad):
+            cu[B + i + 1] = at + i + 1
+            logit_rows.append(at + i)
+        host = {}
         if self.state is not None:
-            pad_slot = self.state.n_slots - 1
-            extra["state_slots"] = torch.tensor([s.state_slot for s, _ in plan] + [pad_slot] * max(0, pad_to - B), dtype=torch.int32)
-        host = {
-            **extra,
-            "ids": torch.tensor(ids, dtype=torch.int32), "positions": torch.tensor(pos, dtype=torch.int32),
-            "slot_map": torch.tensor(slots, dtype=torch.int64), "block_table": bt, "seq_lens": torch.tensor(lens, dtype=torch.int32),
-            "cu_q": torch.tensor(cu, dtype=torch.int32), "logit_rows": torch.tensor(logit_rows, dtype=torch.int64),
-        }
-        return host, max(n for _, n in plan)
+            host["state_slots"] = np.array([s.state_slot for s, _ in plan] + [self.state.n_slots - 1] * pad, np.int32)
+        host.update(ids=ids, positions=pos, slot_map=slots, block_table=bt, seq_lens=lens, cu_q=cu, logit_rows=np.array(logit_rows, np.int64))
+        return {k: torch.from_numpy(v) for k, v in host.items()}, max(n for _, n in plan)
+
+    def _upload(self, host: dict, flat: Optional[torch.Tensor] = None) -> torch.Tensor:
+        """The step's inputs end to end in one buffer on the device (``flat``, or a new one), each at a multiple of 16 bytes: one copy from page-locked
+        memory instead of seven.  The page-locked block comes from PyTorch's caching allocator, which holds it until the copy is done."""
+        on_gpu = self.device.type == "cuda"
+        parts = [(v, _round16(v.numel() * v.element_size())) for v in host.values()]
+        total = sum(n for _, n in parts)
+        stage = torch.empty(total, dtype=torch.uint8, pin_memory=on_gpu)
+        raw, at = stage.numpy(), 0
+        for v, n in parts:
+            b = v.numpy().reshape(-1).view(np.uint8)
+            raw[at:at + b.size] = b
+            self.stats["h2d_bytes"] += b.size
+            at += n
+        if flat is None:
+            return stage.to(self.device, non_blocking=True) if on_gpu else stage
+        return flat.copy_(stage, non_blocking=True)
+
+    @staticmethod
+    def _views(flat: torch.Tensor, host: dict) -> dict:
+        out, at = {}, 0
+        for k, v in host.items():
+            n = v.numel() * v.element_size()
+            out[k] = flat[at:at + n].view(v.dtype).view(v.shape)
+            at += _round16(n)
+        return out
 
     def _to_device(self, host: dict) -> dict:
-        dev = {}
-        for k, v in host.items():
-            if self.device.type == "cuda":
-                v = v.pin_memory()
-            dev[k] = v.to(self.device, non_blocking=True)
-            self.stats["h2d_bytes"] += v.numel() * v.element_size()
-        return dev
+        return self._views(self._upload(host), host)
 
     def _sampling_tensors(self, seqs: list, pad_to: int = 0):
         n = max(len(seqs), pad_to)
@@ -672,9 +690,7 @@ class LLMEngine:
         if g is None:
             g = self._capture(gb, host)
             self._graphs[gb] = g
-        for k, v in host.items():
-            g["in"][k].copy_(v.pin_memory(), non_blocking=True)
-            self.stats["h2d_bytes"] += v.numel() * v.element_size()
+        self._upload(host, g["in"])
         g["graph"].replay()
         from ..ops import cuda as kernels
         kernels._count(g["kernels"])
@@ -695,9 +711,7 @@ class LLMEngine:
         if g is None:
             g = self._capture(n, host, prefill_tokens=n)
             self._graphs[key] = g
-        for k, v in host.items():
-            g["in"][k].copy_(v.pin_memory(), non_blocking=True)
-            self.stats["h2d_bytes"] += v.numel() * v.element_size()
+        self._upload(host, g["in"])
         g["graph"].replay()
         from ..ops import cuda as kernels
         kernels._count(g["kernels"])
@@ -705,15 +719,16 @@ class LLMEngine:
         return g
 
     def _capture(self, gb: int, host: dict, prefill_tokens: int = 0) -> dict:
-        dev = {k: v.to(self.device) for k, v in host.items()}
+        flat = self._upload(host)
+        dev = self._views(flat, host)
         fb = ForwardBatch(dev["ids"], dev["positions"], dev["slot_map"], dev["block_table"], dev["seq_lens"], dev["cu_q"], prefill_tokens or 1,
                           logit_rows=dev["logit_rows"], state_slots=dev.get("state_slots"))
         fwd = (lambda: self.model.forward(fb, self.kv, self.state)) if self.state is not None else (lambda: self.model.forward(fb, self.kv))
         if prefill_tokens:
-            return self._capture_with(fwd, dev, host, argmax=False)
-        return self._capture_with(fwd, dev, host, argmax=True)
+            return self._capture_with(fwd, flat, host, argmax=False)
+        return self._capture_with(fwd, flat, host, argmax=True)
 
-    def _capture_with(self, fwd, dev: dict, host: dict, argmax: bool) -> dict:
+    def _capture_with(self, fwd, flat: torch.Tensor, host: dict, argmax: bool) -> dict:
         post = ops.argmax if argmax else (lambda t: t)
         snap = None
         if self.state is not None:
@@ -748,7 +763,7 @@ class LLMEngine:
                 self.state.restore(sl, sn)
         if self._graph_pool is None:
             self._graph_pool = graph.pool()
-        return {"graph": graph, "in": dev, "out": out, "logits": logits, "kernels": n_kernels}
+        return {"graph": graph, "in": flat, "out": out, "logits": logits, "kernels": n_kernels}
 
     # ------------------------------------------------------------------ convenience
     def generate(self, prompts: list, params: Optional[SamplingParams] = None) -> list:
@@ -757,6 +772,10 @@ class LLMEngine:
         while any(not s.finished for s in seqs):
             self.step()
         return [s.tokens[len(s.prompt):] for s in seqs]
+
+
+def _round16(n: int) -> int:
+    return (n + 15) // 16 * 16
 
 
 def _seed_state(seed: int, seq_id: int, step: int) -> int:
