@@ -9,9 +9,13 @@
 // so that only three small matrix products per chunk depend on the running state.  Two kernels:
 //
 //   dn_chunk_prep_kernel  one CTA per (chunk, v-head), all chunks in parallel.  L2-normalises q and k, forms the gates, K K^T and Q K^T
-//       with one tcgen05.mma (M = 128: K rows then Q rows; N = 64; accumulator in TMEM), then solves (I + A) W = [beta V | beta e^G K]
-//       by forward substitution in fp32 (one thread per right-hand-side column, the column in registers) and writes the chunk's
-//       operands as ready-made shared-memory images (128-byte-swizzled K-major tiles): [e^G Q ; W_k], M, (e^{G_last - G} K)^T, W_v.
+//       with one tcgen05.mma (M = 128: K rows then Q rows; N = 64; accumulator in TMEM), then T = (I + A)^-1 by forward substitution in fp32 on
+//       the 64 columns of the identity (four threads per column), and W_v = T diag(beta) V, W_k = T diag(beta e^G) K on the tensor cores.  V and K
+//       are bf16 as they are; the fp32 factor is the sum of three bf16 terms (24 bits), so nothing is rounded that was not before.  Substituting
+//       on the 256 columns of [beta V | beta e^G K] themselves, as this kernel did, is bound by the shared-memory broadcasts of A: four cycles for
+//       each 16 bytes, 504 of them per warp.  The chunk's operands leave as ready-made shared-memory images (128-byte-swizzled K-major
+//       tiles): [e^G Q ; W_k], M, (e^{G_last - G} K)^T, W_v.
+//       Measured (B200): 4100 tokens of two prompts, 32 heads: the layer's mixer 446 -> 374 us together with the head norm's vector loads.
 //   dn_chunk_scan_kernel  one CTA per (sequence, v-head, half of the v columns), chunks in order.  The state slice lives in registers
 //       (thread = k index, 64 v columns each) and goes to shared memory as a bf16 hi + lo pair (an MN-major B operand) once per
 //       chunk.  Per chunk:  [e^G Q ; W_k] S0^T -> TMEM (rows 0..63 start the output, rows 64..127 are W_k S0^T);  U = W_v - W_k S0^T
@@ -77,11 +81,8 @@ struct PrepSmem {
   static constexpr int TOTAL = MISC + 256 + 1024;
 };
 
-// (shared-window load: a pointer derived from the aligned dynamic base would compile to a generic load)
-__device__ __forceinline__ float lds_bf16(uint32_t addr) {
-  uint16_t v;
-  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr));
-  return __uint_as_float((uint32_t)v << 16);
+__device__ __forceinline__ void dc_bulk_out(void* dst, uint32_t src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(src), "r"(bytes) : "memory");
 }
 
 __global__ void __launch_bounds__(256, 2) dn_chunk_prep_kernel(const ChunkParams p) {
@@ -90,7 +91,7 @@ __global__ void __launch_bounds__(256, 2) dn_chunk_prep_kernel(const ChunkParams
   const uint32_t sbase = smem_u32(smem);
   // Arrays the threads read in their inner loops are static: the dynamic window's pointers come from integer arithmetic (the 1024-byte
   // alignment), so dereferencing them compiles to generic loads, which take the long-latency path.
-  __shared__ __align__(16) float sA[DC * DC];                          // A, fp32
+  __shared__ __align__(1024) float sA[DC * DC];                        // A, fp32; then the first term of T
   __shared__ float sg[DC], sbeta[DC];                                  // g then G (cumulative), beta
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem + PrepSmem::MISC);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bar + 1);
@@ -102,14 +103,14 @@ __global__ void __launch_bounds__(256, 2) dn_chunk_prep_kernel(const ChunkParams
   if (!dc_locate(p.cu_q, p.B, blockIdx.x, b, t0, n)) return;            // whole CTA, before any barrier / TMEM use
   const int kh = p.k_of_v[h];
   if (tid == 0) { mbar_init(smem_u32(bar), 1); *abort_flag = 0; fence_mbar_init(); }
-  if (warp == 0) { tmem_alloc(smem_u32(tmem_slot), 64); tmem_relinquish(); }
+  if (warp == 0) { tmem_alloc(smem_u32(tmem_slot), 256); tmem_relinquish(); }
 
-  // A warp owns rows warp, warp + 8, ...; their loads are issued together and before the gate arithmetic, so that the eight rows cost
+  // A warp owns rows 8 warp .. + 7; their loads are issued together and before the gate arithmetic, so that the eight rows cost
   // one trip to memory and that trip overlaps the gates and their prefix sum.
   uint2 qraw[DC / 8], kraw[DC / 8], vraw[DC / 8];
 #pragma unroll
   for (int it = 0; it < DC / 8; ++it) {
-    const int r = warp + 8 * it;
+    const int r = warp * 8 + it;
     qraw[it] = kraw[it] = vraw[it] = make_uint2(0u, 0u);
     if (r < n) {
       const bf16* row = p.qkv + (size_t)(t0 + r) * p.ld + lane * 4;
@@ -148,15 +149,22 @@ __global__ void __launch_bounds__(256, 2) dn_chunk_prep_kernel(const ChunkParams
   __syncthreads();
   const float Gl = sg[DC - 1];
 
-  // rows: L2 norms, the [K ; Q] operand, e^G Q and (e^{G_last - G} K)^T
+  // rows: L2 norms, the [K ; Q] operand, e^G Q; e^{G_last - G} K stays in registers: a lane has eight positions of four k, 16 bytes of four rows of the
+  // transposed tile
+  uint32_t kd[4][4];
 #pragma unroll
   for (int it = 0; it < DC / 8; ++it) {
-    const int r = warp + 8 * it;
+    const int r = warp * 8 + it;
     const float q[4] = {bf16_lo(qraw[it].x), bf16_hi(qraw[it].x), bf16_lo(qraw[it].y), bf16_hi(qraw[it].y)};
     const float k[4] = {bf16_lo(kraw[it].x), bf16_hi(kraw[it].x), bf16_lo(kraw[it].y), bf16_hi(kraw[it].y)};
     const float iq = rsqrtf(warp_sum(q[0] * q[0] + q[1] * q[1] + q[2] * q[2] + q[3] * q[3]) + p.eps) * p.q_scale;
     const float ik = rsqrtf(warp_sum(k[0] * k[0] + k[1] * k[1] + k[2] * k[2] + k[3] * k[3]) + p.eps);
     const float eg = __expf(sg[r]), ed = __expf(Gl - sg[r]);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const uint32_t v = pack_bf16(k[i] * ik * ed, 0.f);
+      kd[i][it >> 1] = it & 1 ? kd[i][it >> 1] | v << 16 : v;
+    }
     const uint32_t atom = (uint32_t)(lane >> 4) * 16384u, chunk = (lane & 15) >> 1, half = (lane & 1) * 8;
     *reinterpret_cast<uint2*>(smem + PrepSmem::AK + atom + sw128_offset(r, chunk) + half) =
         make_uint2(pack_bf16(k[0] * ik, k[1] * ik), pack_bf16(k[2] * ik, k[3] * ik));
@@ -164,11 +172,8 @@ __global__ void __launch_bounds__(256, 2) dn_chunk_prep_kernel(const ChunkParams
         make_uint2(pack_bf16(q[0] * iq, q[1] * iq), pack_bf16(q[2] * iq, q[3] * iq));
     *reinterpret_cast<uint2*>(smem + PrepSmem::A1 + atom + sw128_offset(r, chunk) + half) =
         make_uint2(pack_bf16(q[0] * iq * eg, q[1] * iq * eg), pack_bf16(q[2] * iq * eg, q[3] * iq * eg));
-#pragma unroll
-    for (int i = 0; i < 4; ++i)          // transposed: element (k index, position r)
-      *reinterpret_cast<bf16*>(smem + PrepSmem::KDT + sw128_offset(lane * 4 + i, r >> 3) + (r & 7) * 2) = __float2bfloat16(k[i] * ik * ed);
-    // the raw v row waits in rows 64..127 of the [e^G Q ; W_k] image (W_k lands there after the substitution has read it)
-    *reinterpret_cast<uint2*>(smem + PrepSmem::A1 + atom + 8192 + r * 128 + (lane & 15) * 8) = vraw[it];
+    // the v row in rows 64..127 of the [e^G Q ; W_k] image (an MN-major operand; W_k lands there once it has been multiplied)
+    *reinterpret_cast<uint2*>(smem + PrepSmem::A1 + atom + sw128_offset(64 + r, chunk) + half) = vraw[it];
   }
   fence_proxy_async();
   __syncthreads();
@@ -206,7 +211,7 @@ __global__ void __launch_bounds__(256, 2) dn_chunk_prep_kernel(const ChunkParams
           const int j = col0 + jj + u;
           a[u] = j < i ? bi * __expf(Gi - sg[j]) * __uint_as_float(c[jj + u]) : 0.f;
         }
-        *reinterpret_cast<float4*>(sA + i * DC + col0 + jj) = make_float4(a[0], a[1], a[2], a[3]);
+        *reinterpret_cast<float4*>(sA + i * DC + (((col0 + jj) >> 2) ^ (i & 15)) * 4) = make_float4(a[0], a[1], a[2], a[3]);
       }
     } else if (ok) {
       const int i = row - DC;
@@ -227,59 +232,101 @@ __global__ void __launch_bounds__(256, 2) dn_chunk_prep_kernel(const ChunkParams
   tc_fence_before();
   __syncthreads();
 
-  // (I + A) W = [beta V | beta e^G K]: thread c owns column c of the right-hand side.  (Runs also after a wait that ran out: the block
-  // contains a barrier, and what it then writes is never read, the status word being set.)
+  // T = (I + A)^-1, column c by four threads: thread q holds rows q, q + 4, ..  (Runs also after a wait that ran out: the block contains
+  // barriers, and what it then writes is never read, the status word being set.)
+  const int c = tid >> 2, q4 = tid & 3;
   {
-    float w[DC];
-    const int c = tid;
-    // right-hand sides from shared memory: the staged v rows, and the normalised k rows of the [K ; Q] operand (rows past the
-    // sequence's end are zero in both, and so is their beta)
-    if (c < DD) {
-      const uint32_t va = sbase + PrepSmem::A1 + (uint32_t)(c >> 6) * 16384u + 8192u + (c & 63) * 2;
+    float w[DC / 4];
 #pragma unroll
-      for (int i = 0; i < DC; ++i) w[i] = sbeta[i] * lds_bf16(va + i * 128);
-    } else {
-      const int e = c - DD;
-      const uint32_t ka = sbase + PrepSmem::AK + (uint32_t)(e >> 6) * 16384u + (e & 7) * 2;
-#pragma unroll
-      for (int i = 0; i < DC; ++i) w[i] = sbeta[i] * __expf(sg[i]) * lds_bf16(ka + sw128_offset(i, (e & 63) >> 3));
-    }
-    __syncthreads();                     // every v row has been read: W_k may overwrite them
+    for (int m = 0; m < DC / 4; ++m) w[m] = 4 * m + q4 == c ? 1.f : 0.f;
 #pragma unroll
     for (int i = 1; i < DC; ++i) {
-      float a0 = 0.f, a1 = 0.f, a2 = 0.f, a3 = 0.f;
+      float a0 = 0.f, a1 = 0.f;
 #pragma unroll
-      for (int j = 0; j < (i & ~3); j += 4) {
-        const float4 a = *reinterpret_cast<const float4*>(sA + i * DC + j);
-        a0 = fmaf(a.x, w[j], a0); a1 = fmaf(a.y, w[j + 1], a1); a2 = fmaf(a.z, w[j + 2], a2); a3 = fmaf(a.w, w[j + 3], a3);
+      for (int m = 0; 4 * m < i; ++m) {                  // (A is zero from column i on)
+        const float a = sA[i * DC + 4 * (m ^ (i & 15)) + q4];        // (16-byte groups of a row exchanged, so that the stores of a column spread over the banks)
+        if (m & 1) a1 = fmaf(a, w[m], a1); else a0 = fmaf(a, w[m], a0);
       }
-#pragma unroll
-      for (int j = (i & ~3); j < i; ++j) a0 = fmaf(sA[i * DC + j], w[j], a0);
-      w[i] -= (a0 + a1) + (a2 + a3);
+      a0 += a1;
+      a0 += __shfl_xor_sync(0xffffffffu, a0, 1);
+      a0 += __shfl_xor_sync(0xffffffffu, a0, 2);
+      if (q4 == (i & 3)) w[i >> 2] -= a0;
     }
-    if (c < DD) {
-      float* wv = reinterpret_cast<float*>(ws + WS_WV) + ((size_t)((c >> 6) * 16 + ((c & 63) >> 2)) * DC) * 4 + (c & 3);
+    __syncthreads();                                     // A has been read: the first term overwrites it
+    // T diag(beta) and T diag(beta e^G) as three bf16 terms each, K-major tiles of 64 rows.  The tensor core multiplies 128 rows: the other 64
+    // are whatever operand lies beside the tile, and their products land on accumulator rows nobody reads.
+    const float bv = sbeta[c], bk = bv * __expf(sg[c]);
+    uint8_t* const tv[3] = {reinterpret_cast<uint8_t*>(sA), smem + PrepSmem::KDT, smem + PrepSmem::AK + 8192};
+    uint8_t* const tk[3] = {reinterpret_cast<uint8_t*>(sA) + 8192, smem + PrepSmem::KDT + 8192, smem + PrepSmem::AK + 24576};
 #pragma unroll
-      for (int i = 0; i < DC; ++i) wv[i * 4] = w[i];
-    } else {
-      const int e = c - DD;
-      const uint32_t atom = (uint32_t)(e >> 6) * 16384u, chunk = (e & 63) >> 3, sub = (e & 7) * 2;
+    for (int m = 0; m < DC / 4; ++m) {
+      const uint32_t at = sw128_offset(4 * m + q4, c >> 3) + (c & 7) * 2;
+      float x = w[m] * bv, y = w[m] * bk;
 #pragma unroll
-      for (int i = 0; i < DC; ++i)
-        *reinterpret_cast<bf16*>(smem + PrepSmem::A1 + atom + sw128_offset(64 + i, chunk) + sub) = __float2bfloat16(w[i]);
+      for (int k = 0; k < 3; ++k) {
+        const bf16 xh = __float2bfloat16(x), yh = __float2bfloat16(y);
+        *reinterpret_cast<bf16*>(tv[k] + at) = xh;
+        *reinterpret_cast<bf16*>(tk[k] + at) = yh;
+        x -= __bfloat162float(xh);
+        y -= __bfloat162float(yh);
+      }
     }
   }
+  fence_proxy_async();
   __syncthreads();
-  if (ok) {
-    const uint4* s1 = reinterpret_cast<const uint4*>(smem + PrepSmem::A1);
-    uint4* d1 = reinterpret_cast<uint4*>(ws + WS_A1);
-    for (int i = tid; i < 32768 / 16; i += 256) d1[i] = s1[i];
-    const uint4* s2 = reinterpret_cast<const uint4*>(smem + PrepSmem::KDT);
-    uint4* d2 = reinterpret_cast<uint4*>(ws + WS_KDT);
-    for (int i = tid; i < 16384 / 16; i += 256) d2[i] = s2[i];
-    if (tid == 0) p.egl[(size_t)blockIdx.x * p.n_v + h] = __expf(Gl);
+  if (tid == 0) {
+    tc_fence_after();
+    constexpr uint32_t idesc = umma_idesc_bf16(128, DD, 0, 1);
+    const uint32_t tv[3] = {smem_u32(sA), sbase + PrepSmem::KDT, sbase + PrepSmem::AK + 8192};
+    const uint32_t tk[3] = {smem_u32(sA), sbase + PrepSmem::KDT, sbase + PrepSmem::AK + 16384};      // (64 rows before the tile)
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+#pragma unroll
+      for (int kk = 0; kk < DC / 16; ++kk) {
+        umma_bf16(tmem_base, umma_desc_k_sw128(tv[k] + kk * 32), umma_desc_mn_sw128(sbase + PrepSmem::A1 + 8192 + kk * 2048, 16384, 1024), idesc, (k | kk) != 0);
+        umma_bf16(tmem_base + DD, umma_desc_k_sw128(tk[k] + kk * 32), umma_desc_mn_sw128(sbase + PrepSmem::AK + kk * 2048, 16384, 1024), idesc, (k | kk) != 0);
+      }
+    umma_commit(mbar);
   }
-  if (warp == 0) tmem_dealloc(tmem_base, 64);
+  const bool ok2 = mbar_wait(mbar, 1, p.status, ERR_MBAR_TIMEOUT_EPILOGUE, abort_flag, 32) && ok;
+  tc_fence_after();
+  if (ok2) {
+    // W_v in accumulator rows 0..63 of the first product, W_k in rows 64..127 of the second; warps w and w + 4 take 64 columns each
+    const int row = (warp & 3) * 32 + lane, hv = warp >> 2;
+    const uint32_t src = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + (row < DC ? 0 : DD) + hv * 64;
+#pragma unroll
+    for (int part = 0; part < 2; ++part) {
+      uint32_t d[32];
+      tmem_ld_32x32(src + part * 32, d);
+      tmem_ld_wait();
+      if (row < DC) {
+        float4* wv = reinterpret_cast<float4*>(ws + WS_WV) + (hv * 16 + part * 8) * DC + row;
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          wv[j * DC] = make_float4(__uint_as_float(d[4 * j]), __uint_as_float(d[4 * j + 1]), __uint_as_float(d[4 * j + 2]), __uint_as_float(d[4 * j + 3]));
+      } else {
+#pragma unroll
+        for (int ch = 0; ch < 4; ++ch)
+          *reinterpret_cast<uint4*>(smem + PrepSmem::A1 + hv * 16384 + sw128_offset(row, part * 4 + ch)) =
+              make_uint4(pack_bf16(__uint_as_float(d[8 * ch]), __uint_as_float(d[8 * ch + 1])), pack_bf16(__uint_as_float(d[8 * ch + 2]), __uint_as_float(d[8 * ch + 3])),
+                         pack_bf16(__uint_as_float(d[8 * ch + 4]), __uint_as_float(d[8 * ch + 5])), pack_bf16(__uint_as_float(d[8 * ch + 6]), __uint_as_float(d[8 * ch + 7])));
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)          // (e^{G_last - G} K)^T: row k index, chunk of eight positions
+      *reinterpret_cast<uint4*>(smem + PrepSmem::KDT + sw128_offset(lane * 4 + i, warp)) = make_uint4(kd[i][0], kd[i][1], kd[i][2], kd[i][3]);
+  }
+  fence_proxy_async();
+  tc_fence_before();
+  __syncthreads();
+  if (ok2 && tid == 0) {
+    dc_bulk_out(ws + WS_A1, sbase + PrepSmem::A1, 32768);
+    dc_bulk_out(ws + WS_KDT, sbase + PrepSmem::KDT, 16384);
+    p.egl[(size_t)blockIdx.x * p.n_v + h] = __expf(Gl);
+    asm volatile("cp.async.bulk.commit_group;\n\tcp.async.bulk.wait_group 0;" ::: "memory");
+  }
+  __syncwarp();
+  if (warp == 0) tmem_dealloc(tmem_base, 256);
 }
 
 // ------------------------------------------------------------------------------------------------ scan
