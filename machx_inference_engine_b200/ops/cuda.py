@@ -527,7 +527,7 @@ def _few_rows_take_gemm(M: int, w: QuantWeight, act: int) -> bool:
     return (M >= 3 and 2 * M * w.K + 16 * min(w.K, 4096) > 190 * 1024) or (M >= 5 and w.N * w.K >= 48 << 20)
 
 
-GEMM_ROWS_MAX = 64        # activation rows per group of the weight-streaming kernel (csrc/cuda/gemm_rows.cu)
+GEMM_ROWS_Q8_MAX = 40     # dense Q8 layers take the weight-streaming kernel (csrc/cuda/gemm_rows.cu) up to this many rows
 
 
 def _takes_rows(x, w: QuantWeight, act: int, row_scale) -> bool:
@@ -535,13 +535,13 @@ def _takes_rows(x, w: QuantWeight, act: int, row_scale) -> bool:
     two rows stay with the GEMV (6144 x 4096: bf16 21.4 -> 22.6, Q8 19.3 -> 23.5) except for gated bf16 and Q8 (28672 x 4096: 104 -> 58, 56 -> 42), which it reads
     once per row; three rows 27.5 -> 23.4 and 25.4 -> 23.4, eight 55 -> 23 and 48 -> 24, forty 38 -> 29 and 64 -> 36.  Above: bf16 48 rows 38 -> 30, 64 rows
     38 -> 34 but 30 -> 33 for 5120 x 2880; matrices of several full waves (from 100 M elements) are already near the memory rate in the tcgen05
-    kernel: 28672 x 4096 33 rows 71 -> 63, 48 rows 71 -> 70, 32768 x 4096 24 rows 68 -> 66, 33 rows 68.6 -> 69.7.  Q8 48 rows 64 -> 32 and 97 -> 76, 64 rows
-    54 -> 47 and 142 -> 106 (there the other kernels decode the weight once), 56 rows of 32768 x 4096 97 -> 104."""
+    kernel: 28672 x 4096 33 rows 71 -> 63, 48 rows 71 -> 70, 32768 x 4096 24 rows 68 -> 66, 33 rows 68.6 -> 69.7.  Q8 40 rows 64 -> 36 and 97 -> 69; 48 rows would
+    still gain (64 -> 32), but between there and DEQUANT_ONCE_MIN_M the values are those of the in-kernel decode that :func:`gemm` gives, bit for bit."""
     M, big = x.shape[0], w.N * w.K >= 100 << 20
     if w.fmt == WFormat.BF16:
         most = 32 if big else 48
     elif w.fmt == WFormat.Q8:
-        most = 48 if big else GEMM_ROWS_MAX
+        most = GEMM_ROWS_Q8_MAX
     else:
         return False
     least = 2 if act_gated(act) else 3
