@@ -74,7 +74,7 @@ def build_host(force: bool = False) -> Path:
 # Kernel sources the layer-list graphs need: no DeltaNet, EXL3, MXFP4 or sharded prefill.  A checkout without the full library
 # can compile just these (``_lib.use_components("core")``); the full library, when it is there, serves every graph.
 COMPONENTS = {
-    "core": ("common", "comm", "elementwise", "gemm_tcgen05", "gemm_rows", "gemv", "gemv_stream", "linear_f32", "attention", "attention_decode", "attention_tc", "mingru", "latent",
+    "core": ("common", "comm", "elementwise", "gemm_tcgen05", "gemm_pair", "gemm_rows", "gemv", "gemv_stream", "linear_f32", "attention", "attention_decode", "attention_tc", "mingru", "latent",
              "latent_tc", "linear_scan", "decay_chunk", "pooled", "rglru", "moe", "sampling"),
 }
 

@@ -498,6 +498,18 @@ def _pick_bn(M: int, N: int, wide: bool = False) -> int:
     return 256 if wide and 1.71 * waves(256) < waves(128) else 128
 
 
+def _takes_pair(M: int, N: int) -> bool:
+    """Whether a bf16 product of more than 128 rows runs on pairs of SMs (``csrc/cuda/gemm_pair.cu``, 256 x 256 tiles, the same values bit for bit): where its
+    waves are shorter.  In units of a wave of 128-row tiles of 64 or 128 columns (which take about as long, 26 us at K = 4096) a wave of 256 columns
+    takes 1.95 and one of pair tiles 1.45 (39 us).  Both sides measured, us, other -> pair: 4096 x 28672 x 4096 742 -> 675, 4096 x 5120 x 2880 138 -> 92, 512 x
+    6144 x 4096 56 -> 46; it stays away from 256 x 4096 x 4096 (32 -> 44, one wave of 64 columns) and 300 x 28672 x 4096 (106 -> 111)."""
+    if M <= 128:
+        return False
+    sms, bn = sm_count(), _pick_bn(M, N, wide=True)
+    waves = -(-(-(-M // 128) * -(-N // bn)) // sms)
+    return 1.45 * -(-(-(-M // 256) * -(-N // 256)) // (sms // 2)) < waves * (1.95 if bn == 256 else 1.0)
+
+
 def _gemm_a(x, w: QuantWeight):
     """Activations in the dtype the tensor-core path of this weight format multiplies in."""
     want = torch.bfloat16
@@ -607,8 +619,12 @@ def linear(x, w: QuantWeight, bias=None, act=ACT_NONE, act_alpha=1.702, act_limi
             _check(lib.mx_dequant_bf16(fmt, p0, p1, p2, p3, C.c_longlong(w.N), w.K, _p(wb), _stream()), "dequant_bf16")
             _count()
             fmt, p0, p1, p2, p3 = int(WFormat.BF16), _p(wb), _vp(0), _vp(0), _vp(0)
-        _check(lib.mx_gemm(_p(xa), fmt, p0, p1, p2, p3, 1, _p(out), out.stride(0), int(out_f32), _p(bias), _p(row_scale), act,
-                           C.c_float(act_alpha), C.c_float(act_limit), M, w.N, w.K, _vp(0), _vp(0), _pick_bn(M, w.N, wide=fmt == int(WFormat.BF16)), _stream()), "gemm")
+        if fmt == int(WFormat.BF16) and _takes_pair(M, w.N):
+            _check(lib.mx_gemm_pair(_p(xa), p0, _p(out), out.stride(0), int(out_f32), _p(bias), _p(row_scale), act, C.c_float(act_alpha), C.c_float(act_limit),
+                                    M, w.N, w.K, _stream()), "gemm_pair")
+        else:
+            _check(lib.mx_gemm(_p(xa), fmt, p0, p1, p2, p3, 1, _p(out), out.stride(0), int(out_f32), _p(bias), _p(row_scale), act,
+                               C.c_float(act_alpha), C.c_float(act_limit), M, w.N, w.K, _vp(0), _vp(0), _pick_bn(M, w.N, wide=fmt == int(WFormat.BF16)), _stream()), "gemm")
     _count()
     return out
 
