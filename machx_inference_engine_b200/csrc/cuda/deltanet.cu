@@ -70,10 +70,18 @@ __global__ void __launch_bounds__(128) conv1d_silu_strip_kernel(const bf16* __re
   if (c >= C) return;
   const int t_lo = blockIdx.y * CONV_STRIP, t_hi = min(T, t_lo + CONV_STRIP);
   float wt[KC][4];                         // [tap][channel]
+  if (KC == 4 && ((uintptr_t)w & 15) == 0) {       // a channel's taps are one vector
 #pragma unroll
-  for (int j = 0; j < KC; ++j)
+    for (int ch = 0; ch < 4; ++ch) {
+      const float4 v = __ldg(reinterpret_cast<const float4*>(w + (size_t)(c + ch) * 4));
+      wt[0][ch] = v.x; wt[1][ch] = v.y; wt[2][ch] = v.z; wt[KC - 1][ch] = v.w;
+    }
+  } else {
 #pragma unroll
-    for (int ch = 0; ch < 4; ++ch) wt[j][ch] = w[(size_t)(c + ch) * KC + j];
+    for (int j = 0; j < KC; ++j)
+#pragma unroll
+      for (int ch = 0; ch < 4; ++ch) wt[j][ch] = w[(size_t)(c + ch) * KC + j];
+  }
   float win[KC][4];                        // win[j] = input at t - (KC - 1) + j
   auto unpack = [](const uint2 raw, float (&o)[4]) {
     o[0] = bf16_lo(raw.x); o[1] = bf16_hi(raw.x); o[2] = bf16_lo(raw.y); o[3] = bf16_hi(raw.y);
@@ -287,47 +295,59 @@ __global__ void __launch_bounds__(DN_THREADS) deltanet_scan_kernel(ScanParams p)
 }
 
 // ------------------------------------------------------------------ gated RMSNorm, z read through a row stride
-// Bound by memory: a lane's loads are independent vectors, issued before the sum of squares (4100 x 32 heads of 128, 134 MB: 49 us with scalar loads in
-// turn, 37 now).  V = 4 needs 16-byte rows of x and w and 8-byte rows of z and y.
-template <int V>
+// Bound by memory: a warp takes four 16-byte vectors of every lane at once (four rows of up to 128 elements, two of up to 256), so that enough bytes are under
+// way.  VPR: vectors of a row per lane, 0: any width and alignment, one row per warp with scalar loads (4100 x 32 heads of 128, 134 MB: 49 us that way, 37 with
+// one vectorised row per warp, MEASURED with four).  The vector forms need 16-byte rows of x and w and 8-byte rows of z and y.
+constexpr int GRN_VECS = 4;
+template <int VPR>
 __global__ void __launch_bounds__(128) gated_rmsnorm_ld_kernel(const float* __restrict__ x, const bf16* __restrict__ z, int z_ld,
                                                                const float* __restrict__ w, bf16* __restrict__ y, int T, int n_h, int hd,
                                                                float eps) {
   pdl_prologue();
-  const int r = blockIdx.x * 4 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (r >= T * n_h) return;
-  const int t = r / n_h, h = r % n_h;
-  const float* xr = x + (size_t)r * hd;
-  const bf16* zr = z + (size_t)t * z_ld + h * hd;
-  if constexpr (V == 4) {                                    // hd <= 256, a multiple of 4
-    float4 xv[2];
-    uint2 zv[2];
-    float ss = 0.f;
+  const int lane = threadIdx.x & 31, warp = blockIdx.x * 4 + (threadIdx.x >> 5);
+  if constexpr (VPR > 0) {
+    constexpr int R = GRN_VECS / VPR;
+    const int r0 = warp * R, rows = T * n_h;
+    float4 xv[R][VPR];
+    uint2 zv[R][VPR];
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const int i = (k * 32 + lane) * 4;
-      xv[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-      zv[k] = make_uint2(0u, 0u);
-      if (i < hd) {
-        xv[k] = *reinterpret_cast<const float4*>(xr + i);
-        zv[k] = *reinterpret_cast<const uint2*>(zr + i);
+    for (int q = 0; q < R; ++q) {
+      const int r = r0 + q, t = r / n_h, h = r - t * n_h;
+#pragma unroll
+      for (int k = 0; k < VPR; ++k) {
+        const int i = (k * 32 + lane) * 4;
+        xv[q][k] = make_float4(0.f, 0.f, 0.f, 0.f);
+        zv[q][k] = make_uint2(0u, 0u);
+        if (r < rows && i < hd) {
+          xv[q][k] = __ldg(reinterpret_cast<const float4*>(x + (size_t)r * hd + i));
+          zv[q][k] = __ldg(reinterpret_cast<const uint2*>(z + (size_t)t * z_ld + h * hd + i));
+        }
       }
     }
-#pragma unroll
-    for (int k = 0; k < 2; ++k) ss += xv[k].x * xv[k].x + xv[k].y * xv[k].y + xv[k].z * xv[k].z + xv[k].w * xv[k].w;
-    ss = warp_sum(ss);
-    const float inv = rsqrtf(ss / hd + eps);
     auto gate = [](float zz) { return zz / (1.f + __expf(-zz)); };
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      const int i = (k * 32 + lane) * 4;
-      if (i >= hd) continue;
-      const float4 g = __ldg(reinterpret_cast<const float4*>(w + i));
-      *reinterpret_cast<uint2*>(y + (size_t)r * hd + i) =
-          make_uint2(pack_bf16(xv[k].x * inv * g.x * gate(bf16_lo(zv[k].x)), xv[k].y * inv * g.y * gate(bf16_hi(zv[k].x))),
-                     pack_bf16(xv[k].z * inv * g.z * gate(bf16_lo(zv[k].y)), xv[k].w * inv * g.w * gate(bf16_hi(zv[k].y))));
+    for (int q = 0; q < R; ++q) {
+      float ss = 0.f;
+#pragma unroll
+      for (int k = 0; k < VPR; ++k) ss += xv[q][k].x * xv[q][k].x + xv[q][k].y * xv[q][k].y + xv[q][k].z * xv[q][k].z + xv[q][k].w * xv[q][k].w;
+      ss = warp_sum(ss);
+      const float inv = rsqrtf(ss / hd + eps);
+#pragma unroll
+      for (int k = 0; k < VPR; ++k) {
+        const int i = (k * 32 + lane) * 4;
+        if (r0 + q >= rows || i >= hd) continue;
+        const float4 g = __ldg(reinterpret_cast<const float4*>(w + i));
+        *reinterpret_cast<uint2*>(y + (size_t)(r0 + q) * hd + i) =
+            make_uint2(pack_bf16(xv[q][k].x * inv * g.x * gate(bf16_lo(zv[q][k].x)), xv[q][k].y * inv * g.y * gate(bf16_hi(zv[q][k].x))),
+                       pack_bf16(xv[q][k].z * inv * g.z * gate(bf16_lo(zv[q][k].y)), xv[q][k].w * inv * g.w * gate(bf16_hi(zv[q][k].y))));
+      }
     }
   } else {
+    const int r = warp;
+    if (r >= T * n_h) return;
+    const int t = r / n_h, h = r % n_h;
+    const float* xr = x + (size_t)r * hd;
+    const bf16* zr = z + (size_t)t * z_ld + h * hd;
     float ss = 0.f;
     for (int i = lane; i < hd; i += 32) ss += xr[i] * xr[i];
     ss = warp_sum(ss);
@@ -384,6 +404,8 @@ MX_HOST_API int mx_gated_rmsnorm_ld(const float* x, const void* z, int z_ld, con
                                     cudaStream_t st) {
   if (T <= 0) return 0;
   const bool vec = hd % 4 == 0 && hd <= 256 && z_ld % 4 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0 && (((uintptr_t)z | (uintptr_t)y) & 7) == 0;
-  launch_pdl(vec ? gated_rmsnorm_ld_kernel<4> : gated_rmsnorm_ld_kernel<1>, dim3((T * n_h + 3) / 4), dim3(128), 0, st, x, (const bf16*)z, z_ld, w, (bf16*)y, T, n_h, hd, eps);
+  auto kern = !vec ? gated_rmsnorm_ld_kernel<0> : hd <= 128 ? gated_rmsnorm_ld_kernel<1> : gated_rmsnorm_ld_kernel<2>;
+  const int per_cta = 4 * (!vec ? 1 : hd <= 128 ? GRN_VECS : GRN_VECS / 2);
+  launch_pdl(kern, dim3((T * n_h + per_cta - 1) / per_cta), dim3(128), 0, st, x, (const bf16*)z, z_ld, w, (bf16*)y, T, n_h, hd, eps);
   return (int)cudaGetLastError();
 }
