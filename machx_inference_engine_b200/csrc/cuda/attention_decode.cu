@@ -577,10 +577,8 @@ __global__ void __launch_bounds__(DA_WARPS * 32, HD == 256 ? 1 : 2) attn_decode_
   cp_async_wait<0>();
 }
 
-// Tickets of the cut groups: zero at load, left at zero by every launch; consecutive launches take the slots in turn, so that launches
-// that overlap (the next kernel of a stream under programmatic dependent launch, other streams) count on different words.
-constexpr int DA_TICKET_SLOTS = 64, DA_MAX_GRID = 512;
-static __device__ int g_decode_tickets[DA_TICKET_SLOTS * DA_MAX_GRID];
+constexpr int DA_MAX_GRID = 512;
+static_assert(DA_MAX_GRID <= CUT_TICKETS, "a counter per CTA");
 
 struct DecodePlan { int nt = 0, q_tile = 0, max_q_tiles = 0; };
 
@@ -635,10 +633,10 @@ MX_HOST_API int mx_attention_decode_scratch(int hd, int B, int n_q, int n_kv, in
 }
 
 // Arguments as in mx_attention_ext / mx_attention_kv8 (k_scale non-null: an int8 cache).  q 4-byte aligned with an even q_ld, cache pages 16-byte
-// aligned, out 8-byte aligned.
+// aligned, out 8-byte aligned.  tickets: see host_util.h.
 MX_HOST_API int mx_attention_decode(const void* q, int q_ld, const void* k_cache, const void* v_cache, const float* k_scale, const float* v_scale,
                                     const int* block_table, const int* seq_lens, const int* cu_q, const float* sinks, const void* gate, int gate_ld,
-                                    const float* q_scale, int q_scale_n, void* out, float* scratch, int B, int Tq, int max_q_len, int n_q, int n_kv, int hd,
+                                    const float* q_scale, int q_scale_n, void* out, float* scratch, int* tickets, int B, int Tq, int max_q_len, int n_q, int n_kv, int hd,
                                     int max_blocks, int block_size, int window, int keep_first, int gate_heads, float scale, float softcap,
                                     cudaStream_t st) {
   if (B <= 0 || Tq <= 0) return 0;
@@ -654,16 +652,7 @@ MX_HOST_API int mx_attention_decode(const void* q, int q_ld, const void* k_cache
   p.keep_first = window > 0 ? keep_first : 0;
   p.B = B; p.n_q = n_q; p.n_kv = n_kv; p.max_blocks = max_blocks; p.block_size = block_size; p.q_tile = pl.q_tile; p.max_q_tiles = pl.max_q_tiles;
   p.window = window; p.scale = scale; p.softcap = softcap;
-  static std::atomic<int*> base[64];
-  static std::atomic<unsigned> turn{0};
-  const int dev = DeviceOnce::ordinal();
-  int* tickets = base[dev].load(std::memory_order_acquire);
-  if (!tickets) {
-    void* a = nullptr;
-    if (cudaGetSymbolAddress(&a, g_decode_tickets) != cudaSuccess) return -115;
-    base[dev].store(tickets = (int*)a, std::memory_order_release);
-  }
-  p.tickets = tickets + (size_t)(turn.fetch_add(1) % DA_TICKET_SLOTS) * DA_MAX_GRID;
+  p.tickets = tickets;
 #define MX_DA(HD_, NT_) (k_scale ? launch_decode<HD_, NT_, true>(p, scratch, st) : launch_decode<HD_, NT_, false>(p, scratch, st))
   if (hd == 64) return pl.nt == 1 ? MX_DA(64, 1) : pl.nt == 2 ? MX_DA(64, 2) : MX_DA(64, 4);
   if (hd == 128) return pl.nt == 1 ? MX_DA(128, 1) : pl.nt == 2 ? MX_DA(128, 2) : MX_DA(128, 4);

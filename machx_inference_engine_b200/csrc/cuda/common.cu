@@ -92,6 +92,19 @@ MX_HOST_API int mx_status_read_and_clear() {
   return v;
 }
 
+MX_HOST_API int mx_cut_tickets() { return mx::CUT_TICKETS; }
+
+// Identity of the graph capture that `st` takes part in, 0: none.
+MX_HOST_API unsigned long long mx_capture_id(cudaStream_t st) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  if (cudaStreamGetCaptureInfo(st, &status, &id) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  return status == cudaStreamCaptureStatusActive ? id : 0;
+}
+
 MX_HOST_API int mx_sm_count() { return mx::sm_count(); }
 
 MX_HOST_API const char* mx_cuda_last_error() {

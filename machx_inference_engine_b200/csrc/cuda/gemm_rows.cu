@@ -33,6 +33,7 @@ constexpr int GR_ROWS = 128;             // weight rows per tile
 constexpr int GR_WARPS = 4;
 constexpr int GR_MAX_ENTRIES = 1024;     // groups of activation rows of a launch
 constexpr int GR_MAX_GRID = 512;
+static_assert(GR_MAX_GRID * GR_WARPS <= CUT_TICKETS, "a counter per warp");
 
 struct GemmRowsParams {
   int M, N, K, n_tiles, k_steps, chunk;  // chunk: activation rows per group (at most 8 NT)
@@ -477,10 +478,6 @@ __global__ void __launch_bounds__(GemmRowsShape<Q8, NT>::WARPS * 32 + 32, 2) gem
   __syncthreads();
 }
 
-// tickets of the cut tiles: zero at load and after every launch; consecutive launches take the slots in turn (launches may overlap)
-constexpr int GR_TICKET_SLOTS = 64;
-static __device__ int g_rows_tickets[GR_TICKET_SLOTS * GR_MAX_GRID * GR_WARPS];
-
 template <bool Q8, int NT> static int launch_rows(const CUtensorMap& tw, const CUtensorMap& tx, const CUtensorMap& td, const GemmRowsParams& p, cudaStream_t st) {
   using S = GemmRowsShape<Q8, NT>;
   auto kern = gemm_rows_kernel<Q8, NT>;
@@ -510,10 +507,11 @@ MX_HOST_API int mx_gemm_rows_scratch(int rows) {
 
 // C[M, N (/2 when gated)] = A[M,K] W[(E,) N, K]^T (+ bias, activation, row scale).  wfmt bf16 or Q8 (w1: scales, rows padded to 16 bytes).  Dense: M <= 64 and
 // tile_expert null.  Grouped: A is packed in 128-row tiles (tile_expert, tile_valid, num_tiles on the device, at most max_tiles <= 1024 of them), taken in
-// groups of `chunk` rows; rows past a tile's live ones are not written.  out_kind 0 bf16, 1 fp32, 2 fp16.
+// groups of `chunk` rows; rows past a tile's live ones are not written.  tickets: see host_util.h.  out_kind 0 bf16, 1 fp32, 2 fp16.
 MX_HOST_API int mx_gemm_rows(const void* a, int wfmt, const void* w0, const void* w1, int n_experts, void* c, int ldc, int out_kind, const float* bias,
                              const float* row_scale, int act, float act_alpha, float act_limit, int M, int N, int K, const int* tile_expert,
-                             const int* tile_valid, const int* num_tiles, int max_tiles, int chunk, float* scratch, cudaStream_t st) {
+                             const int* tile_valid, const int* num_tiles, int max_tiles, int chunk, float* scratch, int* tickets,
+                             cudaStream_t st) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   const bool q8 = wfmt == WF_Q8;
   if ((!q8 && wfmt != WF_BF16) || K % 8 || (q8 && K % 32)) return -101;
@@ -526,16 +524,7 @@ MX_HOST_API int mx_gemm_rows(const void* a, int wfmt, const void* w0, const void
   p.C = c; p.ldc = ldc; p.out_f32 = out_kind; p.bias = bias; p.row_scale = row_scale; p.act = act; p.act_alpha = act_alpha; p.act_limit = act_limit;
   p.tile_expert = tile_expert; p.tile_valid = tile_valid; p.num_tiles = num_tiles; p.max_tiles = max_tiles; p.part = scratch; p.status = status_word();
   if ((long long)(tile_expert ? (long long)max_tiles * ((128 + chunk - 1) / chunk) * 21 : 1) * p.n_tiles * p.k_steps > 0x7fffffffll) return -106;
-  static std::atomic<int*> base[64];
-  static std::atomic<unsigned> turn{0};
-  const int dev = DeviceOnce::ordinal();
-  int* tickets = base[dev].load(std::memory_order_acquire);
-  if (!tickets) {
-    void* addr = nullptr;
-    if (cudaGetSymbolAddress(&addr, g_rows_tickets) != cudaSuccess) return -115;
-    base[dev].store(tickets = (int*)addr, std::memory_order_release);
-  }
-  p.tickets = tickets + (size_t)(turn.fetch_add(1) % GR_TICKET_SLOTS) * (GR_MAX_GRID * GR_WARPS);
+  p.tickets = tickets;
   CUtensorMap tw, tx, td;
   {
     // int8 codes travel as two-byte elements: the tile is bytes either way

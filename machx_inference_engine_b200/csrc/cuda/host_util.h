@@ -23,6 +23,9 @@ int make_tmap_bf16(CUtensorMap* out, const void* base, int rank, const uint64_t*
                    const uint32_t* box, int swizzle128);
 int make_tmap_bytes(CUtensorMap* out, const void* base, uint64_t row_bytes, uint64_t rows, uint64_t row_stride, uint32_t box_bytes, uint32_t box_rows);
 bool pdl_enabled();
+// Counters with which the CTAs of a launch agree who arrives last at a cut piece of work.  The caller passes CUT_TICKETS zeroed words that no other launch
+// counts on at the same time; every launch leaves them at zero again.
+constexpr int CUT_TICKETS = 2048;
 
 // Kernel launch with the programmatic-dependent-launch attribute (see pdl_* in common.cuh).
 template <typename... KArgs, typename... Args>

@@ -7,6 +7,7 @@ from __future__ import annotations
 
 import ctypes as C
 import math
+import threading
 from typing import Optional
 
 import torch
@@ -52,10 +53,49 @@ def _count(n=1):
     _launch_count += n
 
 
+# Counters of cut pieces of work (csrc/cuda/host_util.h): zeroed words that launches which may overlap do not share, and that every launch leaves at zero.
+# Launches of one stream follow one another, so a stream has one array.  A capture zeroes arrays of its own, one per stream that takes part, by a node of
+# the graph, in memory of the graph's pool: the array may be given back as soon as nothing is captured any more, since a block that the pool reuses is
+# used by later work of the same stream, and a replay zeroes it again.
+STREAM_TICKETS_MAX = 64
+_tickets_lock = threading.Lock()
+_stream_tickets: dict = {}          # (device, stream) -> (array, its pointer, the stream)
+_capture_tickets: dict = {}         # (device, stream, capture) -> the same
+
+
+def _tickets(device):
+    """(array, its pointer, the stream) for a launch on the current stream of ``device``; the caller keeps the tuple until it has launched."""
+    s = torch._C._cuda_getCurrentRawStream(device.index)
+    key = (device.index, s) if s != 2 else (device.index, s, threading.get_ident())      # (handle 2: every thread's own default stream)
+    capturing = torch.cuda.is_current_stream_capturing()
+    if not capturing and not _capture_tickets:
+        t = _stream_tickets.get(key)
+        if t is not None:
+            return t
+    with _tickets_lock:
+        table, capture = _stream_tickets, None
+        if capturing:
+            lib = _lib.cuda()
+            lib.mx_capture_id.restype = C.c_ulonglong
+            table, capture = _capture_tickets, lib.mx_capture_id(_vp(s))
+            key += (capture,)
+        for k in [k for k in _capture_tickets if k[-1] != capture]:
+            del _capture_tickets[k]
+        t = table.get(key)
+        if t is None:
+            array = torch.zeros(_lib.cuda().mx_cut_tickets(), dtype=torch.int32, device=device)
+            t = table[key] = (array, _p(array), _vp(s))
+            if len(_stream_tickets) > STREAM_TICKETS_MAX:
+                del _stream_tickets[next(iter(_stream_tickets))]
+        return t
+
+
 def check_status():
     """Synchronise and raise if any kernel recorded a bounded-wait timeout or bad argument."""
     v = _lib.cuda().mx_status_read_and_clear()
     if v:
+        with _tickets_lock:                  # a launch that gave up may have left its counters in the middle
+            _stream_tickets.clear()
         names = {1: "TMA producer wait", 2: "MMA wait", 3: "epilogue wait", 4: "dequant producer wait", 5: "peer flag wait",
                  6: "bad argument", 7: "softmax wait"}
         raise KernelError(f"kernel status {v}: {names.get(v, 'unknown')} ran out of its time limit")
@@ -576,10 +616,11 @@ def _gemm_rows(x, w: QuantWeight, out, out_kind, bias, row_scale, act, act_alpha
     allocation: stream-ordered, of the graph's own pool under capture."""
     lib = _lib.cuda()
     scratch = torch.empty(lib.mx_gemm_rows_scratch(chunk), dtype=torch.float32, device=x.device)
+    tickets = _tickets(x.device)
     te, tv, nt = tiles if tiles is not None else (None, None, None)
     _check(lib.mx_gemm_rows(_p(x), int(w.fmt), _p(w.p0), _p(w.p1), w.E, _p(out), out.stride(0), out_kind, _p(bias), _p(row_scale), act, C.c_float(act_alpha),
                             C.c_float(act_limit), x.shape[0], w.N, w.K, _p(te), _p(tv), _p(nt), 0 if te is None else te.numel(), int(chunk), _p(scratch),
-                            _stream()), "gemm_rows")
+                            tickets[1], tickets[2]), "gemm_rows")
 
 
 def linear(x, w: QuantWeight, bias=None, act=ACT_NONE, act_alpha=1.702, act_limit=7.0, out_f32=False, row_scale=None, out=None):
@@ -865,12 +906,13 @@ def _attention_decode(q, k_cache, v_cache, block_table, seq_lens, cu_q, max_q_le
         assert q_scale is None and gate is None and not keep_first and q.is_contiguous(), "the int8 cache has no gated / position-scaled form"
     ks, vs = kv_scales if kv_scales is not None else (None, None)
     scratch = torch.empty(scratch_floats, dtype=torch.float32, device=q.device)
+    tickets = _tickets(q.device)
     out = torch.empty(Tq, n_q, hd, dtype=torch.bfloat16, device=q.device)
     _check(_lib.cuda().mx_attention_decode(_p(q), _q_rows(q), _p(k_cache), _p(v_cache), _p(ks), _p(vs), _p(block_table), _p(seq_lens), _p(cu_q), _p(sinks),
                                            _p(gate), 0 if gate is None else gate.stride(0), _p(q_scale), 0 if q_scale is None else q_scale.numel(), _p(out),
-                                           _p(scratch), seq_lens.numel(), Tq, int(max_q_len), n_q, k_cache.shape[1], hd, block_table.shape[1],
+                                           _p(scratch), tickets[1], seq_lens.numel(), Tq, int(max_q_len), n_q, k_cache.shape[1], hd, block_table.shape[1],
                                            k_cache.shape[2], int(window), int(keep_first), int(gate is not None and gate.shape[1] == n_q), C.c_float(scale),
-                                           C.c_float(softcap), _stream()), "attention_decode")
+                                           C.c_float(softcap), tickets[2]), "attention_decode")
     _count()
     return out
 
