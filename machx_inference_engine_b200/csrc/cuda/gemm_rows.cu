@@ -10,6 +10,9 @@
 //     stages; four warps own 32 weight rows each and never wait for each other;
 //   * int8 codes go from the swizzled tile through ldmatrix to registers and are widened to bf16 exactly (three instructions per pair); each
 //     32-element block is summed on its own and scaled in fp32, so the weights are not rounded to bf16;
+//   * up to 8 rows of bf16, where the GEMVs of fp32 additions are the alternative: the tensor cores cut a running sum off where an addition rounds (4096
+//     x 4096, error against 64 bits 4.0e-7 that way, 0.87e-7 in the GEMV), so every instruction's 16 products are summed on their own, and the
+//     sums are added in fp32 with the rounding errors carried along (0.72e-7, in the same time);
 //   * the work is the list of (group of rows, 128 weight rows, K step) laid end to end, of which every CTA takes an equal run.  A
 //     tile that is cut leaves fp32 partials (at most two per CTA); the warp that arrives last adds them in the order of the CTAs.
 // A gated pair (16 gate rows, then 16 up rows) lies in one lane's accumulators.
@@ -74,6 +77,12 @@ template <int SEL> __device__ __forceinline__ uint32_t gr_s8_pair(uint32_t w) {
   const uint32_t x = (t & 0x007f007fu) | 0x43004300u, y = (t & 0x00800080u) | 0x43004300u;
   const __nv_bfloat162 d = __hsub2(*reinterpret_cast<const __nv_bfloat162*>(&x), *reinterpret_cast<const __nv_bfloat162*>(&y));
   return *reinterpret_cast<const uint32_t*>(&d);
+}
+// sum += v, with what the rounded sums before it have lost
+__device__ __forceinline__ void add_exact(float& sum, float& lost, float v) {
+  const float y = v - lost, r = sum + y, e = (r - sum) - y;
+  lost = fabsf(e) < INFINITY ? e : 0.f;                      // (an infinite sum stays one)
+  sum = r;
 }
 __device__ __forceinline__ uint32_t gr_lds32(uint32_t addr) {
   uint32_t v;
@@ -276,6 +285,7 @@ __global__ void __launch_bounds__(GemmRowsShape<Q8, NT>::WARPS * 32 + 32, 2) gem
         for (int j = 0; j < NT; ++j)
 #pragma unroll
           for (int i = 0; i < 4; ++i) acc[m][j][i] = 0.f;
+      float lost[2][4] = {};                                 // (bf16, NT = 1)
       // the K steps, over NL live column groups: a count the compiler knows, so that a step is one straight run of instructions
       auto steps = [&](auto live) {
         constexpr int NL = decltype(live)::value;
@@ -283,6 +293,7 @@ __global__ void __launch_bounds__(GemmRowsShape<Q8, NT>::WARPS * 32 + 32, 2) gem
           if (!(ok = mbar_wait(bar_full + 8 * s, ph, p.status, ERR_MBAR_TIMEOUT_MMA, abort_flag))) break;
           const uint32_t st = base + s * S::STAGE;
           if constexpr (!Q8) {
+            float sum[2][2][4];                              // (NT = 1)
   #pragma unroll
             for (int kk = 0; kk < 4; ++kk) {
               uint32_t a[2][4], b[NL][2];
@@ -298,8 +309,22 @@ __global__ void __launch_bounds__(GemmRowsShape<Q8, NT>::WARPS * 32 + 32, 2) gem
   #pragma unroll
               for (int m = 0; m < 2; ++m)
   #pragma unroll
-                for (int j = 0; j < NL; ++j)
-                  gr_mma(acc[m][j], a[m], b[j][0], b[j][1]);
+                for (int j = 0; j < NL; ++j) {
+                  if constexpr (NT > 1) {
+                    gr_mma(acc[m][j], a[m], b[j][0], b[j][1]);
+                  } else {                                   // 16 products on their own; the four of a step meet in pairs
+                    float t[4];
+                    gr_mma_zero(t, a[m], b[j][0], b[j][1]);
+  #pragma unroll
+                    for (int i = 0; i < 4; ++i) sum[m][kk >> 1][i] = kk & 1 ? sum[m][kk >> 1][i] + t[i] : t[i];
+                  }
+                }
+            }
+            if constexpr (NT == 1) {                         // and join the running sum, whose rounding errors are carried along
+  #pragma unroll
+              for (int m = 0; m < 2; ++m)
+  #pragma unroll
+                for (int i = 0; i < 4; ++i) add_exact(acc[m][0][i], lost[m][i], sum[m][0][i] + sum[m][1][i]);
             }
           } else {
             uint32_t sd = st + S::W_BYTES + S::X_BYTES + (wr * 32 + g) * 16 + ((first + k) & 1) * 8 + kh * 4, sx = st;
@@ -411,17 +436,34 @@ __global__ void __launch_bounds__(GemmRowsShape<Q8, NT>::WARPS * 32 + 32, 2) gem
 #pragma unroll
           for (int j = 0; j < NT; ++j)
 #pragma unroll
-            for (int i = 0; i < 4; ++i) acc[m][j][i] = 0.f;
-        for (int c = c0; c <= c1; ++c) {
-          const float4* src = slab(c);
+            for (int i = 0; i < 4; ++i) acc[m][j][i] = lost[m][i] = 0.f;
+        if constexpr (!Q8 && NT == 1) {                        // four parts at a time, in pairs
+          for (int c = c0; c <= c1; c += 4) {
+            float4 v[4][2];
 #pragma unroll
-          for (int m = 0; m < 2; ++m)
+            for (int i = 0; i < 4; ++i)
 #pragma unroll
-            for (int j = 0; j < NT; ++j)
-              if (j < nt_live) {
-                const float4 v = __ldcg(src + (m * NT + j) * 32);
-                acc[m][j][0] += v.x; acc[m][j][1] += v.y; acc[m][j][2] += v.z; acc[m][j][3] += v.w;
-              }
+              for (int m = 0; m < 2; ++m) v[i][m] = c + i <= c1 ? __ldcg(slab(c + i) + m * 32) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int m = 0; m < 2; ++m) {
+              add_exact(acc[m][0][0], lost[m][0], (v[0][m].x + v[1][m].x) + (v[2][m].x + v[3][m].x));
+              add_exact(acc[m][0][1], lost[m][1], (v[0][m].y + v[1][m].y) + (v[2][m].y + v[3][m].y));
+              add_exact(acc[m][0][2], lost[m][2], (v[0][m].z + v[1][m].z) + (v[2][m].z + v[3][m].z));
+              add_exact(acc[m][0][3], lost[m][3], (v[0][m].w + v[1][m].w) + (v[2][m].w + v[3][m].w));
+            }
+          }
+        } else {
+          for (int c = c0; c <= c1; ++c) {
+            const float4* src = slab(c);
+#pragma unroll
+            for (int m = 0; m < 2; ++m)
+#pragma unroll
+              for (int j = 0; j < NT; ++j)
+                if (j < nt_live) {
+                  const float4 v = __ldcg(src + (m * NT + j) * 32);
+                  acc[m][j][0] += v.x; acc[m][j][1] += v.y; acc[m][j][2] += v.z; acc[m][j][3] += v.w;
+                }
+          }
         }
       } else {
         u = at.start + p.k_steps * at.cost;

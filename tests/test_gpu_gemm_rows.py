@@ -107,3 +107,24 @@ def test_launches_on_two_streams_and_in_a_graph_do_not_share_state():
             other = product(x, w, True)
     torch.cuda.synchronize()
     assert torch.equal(got, want) and torch.equal(other, want)
+
+
+@pytest.mark.parametrize("M", [3, 5, 8])
+@pytest.mark.parametrize("N,Kd", [(6144, 4096), (8192, 2880), (5120, 14336)])
+def test_few_rows_in_fp32_lose_nothing_to_the_tensor_cores(M, N, Kd):
+    """Sums of 16 products are cut off by 2^-23 of themselves at most and joined with compensation: with independent terms their errors come to no more
+    than 2^-23 of the result, rounding included 2^-22.  A running sum kept in the tensor core is cut off K / 16 times: 4e-7 to 3e-6 at these sizes."""
+    x = torch.randn(M, Kd, generator=torch.Generator().manual_seed(M)).to("cuda:0", torch.bfloat16)
+    w = weight(WFormat.BF16, N, Kd, seed=N)
+    assert rel(product(x, w, True), x.double() @ values(w)[0].T) < 2.0 ** -22
+    assert rel(ops.linear(x, w, out_f32=True), x.double() @ values(w)[0].T) < 2.0 ** -22
+
+
+def test_infinite_sums_stay_infinite():
+    w = from_dense(torch.rand(1, 6144, 4096, generator=torch.Generator().manual_seed(5)) + 0.5, WFormat.BF16).to("cuda:0")
+    x = torch.ones(4, 4096, dtype=torch.bfloat16, device="cuda:0")
+    x[0, 7] = float("inf")
+    x[1, ::3] = 3e38
+    x[2, 4000] = float("nan")
+    got = product(x, w, True)
+    assert bool(torch.isposinf(got[:2]).all()) and bool(got[2].isnan().all()) and rel(got[3], x[3].double() @ values(w)[0].T) < 2.0 ** -21
