@@ -100,6 +100,14 @@ template <int SEL> __device__ __forceinline__ uint32_t s8_pair_bf16(uint32_t w) 
   return *reinterpret_cast<const uint32_t*>(&d);
 }
 
+// Tiles per CTA.  An equal share, but not so little that merging costs more than it saves: a partial is read back at about an eighth of a tile's time,
+// so n / per partials and per tiles balance at per = sqrt(n / 8).
+__host__ __device__ inline int decode_run(int total, int grid, int most) {
+  int per = total > grid ? (total - 1) / grid + 1 : 1;
+  while ((long long)per * per * 8 < most) ++per;
+  return per;
+}
+
 template <int HD, int NT, bool KV8> struct DecodeShape {
   static constexpr int RB = HD * (KV8 ? 1 : 2);                         // bytes of a cache row
   static constexpr int SK = RB <= 128 ? 32 : 16;                        // keys per warp step
@@ -165,10 +173,7 @@ __global__ void __launch_bounds__(DA_WARPS * 32, HD == 256 ? 1 : 2) attn_decode_
     for (int w = 0; w < DA_WARPS; ++w) most = max(most, s_red[1][w]);
   }
   const int total = s_pre[entries] * p.n_kv;
-  // An equal share, but not so little that merging costs more than it saves: a partial is read back at about an eighth of a tile's time, so
-  // n / per partials and per tiles balance at per = sqrt(n / 8).
-  int per = max(1, (total + (int)gridDim.x - 1) / (int)gridDim.x);
-  while (per * per * 8 < most) ++per;
+  const int per = decode_run(total, (int)gridDim.x, most);
   const int my0 = blockIdx.x * per, my1 = min(total, my0 + per);
   if (my0 >= total) return;
   int e_first = 0;
@@ -631,6 +636,8 @@ MX_HOST_API int mx_attention_decode_scratch(int hd, int B, int n_q, int n_kv, in
   if (!decode_plan(hd, B, n_q, n_kv, max_q_len, pl)) return 0;
   return DA_MAX_GRID * 2 * 8 * pl.nt * (hd + 2);
 }
+
+MX_HOST_API int mx_attention_decode_run(int total, int grid, int most) { return decode_run(total, grid, most); }
 
 // Arguments as in mx_attention_ext / mx_attention_kv8 (k_scale non-null: an int8 cache).  q 4-byte aligned with an even q_ld, cache pages 16-byte
 // aligned, out 8-byte aligned.  tickets: see host_util.h.

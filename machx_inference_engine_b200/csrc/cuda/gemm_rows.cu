@@ -111,6 +111,16 @@ template <bool Q8, int NT> struct GemmRowsShape {
   static constexpr int SMEM = NST * STAGE + XCH + 1024;
 };
 
+// Units of work per CTA.  An equal share each, but cutting a tile into ever shorter runs costs the last warp the partials' read: about NT / 15 of a step's
+// time per part, so runs are at least sqrt(steps NT / 15) long; and no CTA lies without a step between two others.
+__host__ __device__ inline int rows_run(int total, int grid, int steps_nt, int cost) {
+  int per = (total - 1) / grid + 1;
+  if (per < cost) per = cost;
+  while ((long long)per * per * 15 < steps_nt) ++per;
+  return per;
+}
+__host__ __device__ inline int rows_cost(bool weighted, int rows) { return weighted ? 5 + 2 * ((rows + 7) / 8) : 1; }
+
 template <bool Q8, int NT>
 __global__ void __launch_bounds__(GemmRowsShape<Q8, NT>::WARPS * 32 + 32, 2) gemm_rows_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant__ CUtensorMap tm_x,
                                                                           const __grid_constant__ CUtensorMap tm_d, const GemmRowsParams p) {
@@ -140,7 +150,7 @@ __global__ void __launch_bounds__(GemmRowsShape<Q8, NT>::WARPS * 32 + 32, 2) gem
 
   // ---- the list of work: groups of activation rows x weight tiles x K steps.  A step of a group costs `cost` units: with int8 codes the
   // instructions grow with the live column groups (about 5 + 2 per group), bf16 steps are bound by their bytes.
-  auto cost = [&](int rows) { return Q8 && grouped ? 5 + 2 * ((rows + 7) / 8) : 1; };
+  auto cost = [&](int rows) { return rows_cost(Q8 && grouped, rows); };
   int units = 1, live_tiles = 0;
   if (grouped) {
     pdl_wait();
@@ -172,10 +182,7 @@ __global__ void __launch_bounds__(GemmRowsShape<Q8, NT>::WARPS * 32 + 32, 2) gem
     __syncthreads();
   }
   const int steps_of = p.n_tiles * p.k_steps, total = units * steps_of;       // (of one unit of cost)
-  // An equal share each, but cutting a tile into ever shorter runs costs the last warp the partials' read: about NT / 15 of a step's time per
-  // part, so runs are at least sqrt(steps NT / 15) long.
-  int per = max(cost(p.chunk), (total + (int)gridDim.x - 1) / (int)gridDim.x);      // (no CTA between two others without a step)
-  while (per * per * 15 < p.k_steps * NT) ++per;
+  const int per = rows_run(total, (int)gridDim.x, p.k_steps * NT, cost(p.chunk));
   const int my0 = min(total, (int)blockIdx.x * per), my1 = min(total, my0 + per);
 
   // A run is walked step by step: position `at` (in units of cost) of the step's start.  A step belongs to the CTA in whose run it starts.
@@ -547,8 +554,17 @@ MX_HOST_API int mx_gemm_rows_scratch(int rows) {
   return GR_MAX_GRID * 2 * GR_ROWS * 8 * rows_nt(rows);
 }
 
+// Whether mx_gemm_rows takes a bank of experts: its kernel counts the tiles in shared memory and the work in 32 bits.
+MX_HOST_API int mx_gemm_rows_takes(int wfmt, int max_tiles, int chunk, int N, int K) {
+  if (chunk < 1 || chunk > 64 || max_tiles > GR_MAX_ENTRIES) return 0;
+  const long long units = (128 + chunk - 1) / chunk * rows_cost(wfmt == WF_Q8, chunk);
+  const int ks = wfmt == WF_Q8 ? 128 : 64;
+  return units * max_tiles * ((N + GR_ROWS - 1) / GR_ROWS) * ((K + ks - 1) / ks) < 1ll << 30;
+}
+MX_HOST_API int mx_gemm_rows_run(int total, int grid, int steps_nt, int cost) { return rows_run(total, grid, steps_nt, cost); }
+
 // C[M, N (/2 when gated)] = A[M,K] W[(E,) N, K]^T (+ bias, activation, row scale).  wfmt bf16 or Q8 (w1: scales, rows padded to 16 bytes).  Dense: M <= 64 and
-// tile_expert null.  Grouped: A is packed in 128-row tiles (tile_expert, tile_valid, num_tiles on the device, at most max_tiles <= 1024 of them), taken in
+// tile_expert null.  Grouped: A is packed in 128-row tiles (tile_expert, tile_valid, num_tiles on the device, at most max_tiles of them: mx_gemm_rows_takes), taken in
 // groups of `chunk` rows; rows past a tile's live ones are not written.  tickets: see host_util.h.  out_kind 0 bf16, 1 fp32, 2 fp16.
 MX_HOST_API int mx_gemm_rows(const void* a, int wfmt, const void* w0, const void* w1, int n_experts, void* c, int ldc, int out_kind, const float* bias,
                              const float* row_scale, int act, float act_alpha, float act_limit, int M, int N, int K, const int* tile_expert,
@@ -558,14 +574,13 @@ MX_HOST_API int mx_gemm_rows(const void* a, int wfmt, const void* w0, const void
   const bool q8 = wfmt == WF_Q8;
   if ((!q8 && wfmt != WF_BF16) || K % 8 || (q8 && K % 32)) return -101;
   if (act_gated(act) && N % 32) return -104;
-  if (chunk < 1 || chunk > 64 || (tile_expert ? (max_tiles > GR_MAX_ENTRIES || !tile_valid || !num_tiles || row_scale) : M > chunk)) return -106;
+  if (chunk < 1 || chunk > 64 || (tile_expert ? (!mx_gemm_rows_takes(wfmt, max_tiles, chunk, N, K) || !tile_valid || !num_tiles || row_scale) : M > chunk)) return -106;
   if (((uintptr_t)a | (uintptr_t)w0 | (uintptr_t)w1 | (uintptr_t)scratch) & 15) return -114;
   const int nt = rows_nt(chunk), ks = q8 ? 128 : 64;
   GemmRowsParams p;
   p.M = M; p.N = N; p.K = K; p.n_tiles = (N + GR_ROWS - 1) / GR_ROWS; p.k_steps = (K + ks - 1) / ks; p.chunk = chunk;
   p.C = c; p.ldc = ldc; p.out_f32 = out_kind; p.bias = bias; p.row_scale = row_scale; p.act = act; p.act_alpha = act_alpha; p.act_limit = act_limit;
   p.tile_expert = tile_expert; p.tile_valid = tile_valid; p.num_tiles = num_tiles; p.max_tiles = max_tiles; p.part = scratch; p.status = status_word();
-  if ((long long)(tile_expert ? (long long)max_tiles * ((128 + chunk - 1) / chunk) * 21 : 1) * p.n_tiles * p.k_steps > 0x7fffffffll) return -106;
   p.tickets = tickets;
   CUtensorMap tw, tx, td;
   {

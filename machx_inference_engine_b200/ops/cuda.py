@@ -781,7 +781,7 @@ def grouped_linear(xp, w: QuantWeight, tile_expert, num_tiles, bias=None, act=AC
     out = torch.empty(P, n_out, dtype=odt, device=xp.device)
     fmt, p0, p1, p2, p3 = _planes(w)
     xp = _gemm_a(xp, w)
-    if chunk and tile_valid is not None and w.fmt in (WFormat.BF16, WFormat.Q8) and tile_expert.numel() <= 1024:
+    if chunk and tile_valid is not None and w.fmt in (WFormat.BF16, WFormat.Q8) and _lib.cuda().mx_gemm_rows_takes(fmt, tile_expert.numel(), chunk, w.N, w.K):
         _gemm_rows(xp, w, out, _out_kind(odt), bias, None, act, act_alpha, act_limit, chunk, tiles=(tile_expert, tile_valid, num_tiles))
         _count()
         return out
