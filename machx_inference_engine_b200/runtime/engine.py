@@ -480,6 +480,8 @@ class LLMEngine:
             s0 = seq.n_computed
             if len(seq.blocks) > mb:
                 raise ContextLengthExceeded("sequence outgrew the block table")
+            if s0 + n > len(seq.blocks) * KV_BLOCK:        # (the table's other entries are the null block, which padding writes to)
+                raise IndexError("sequence without a KV block for its last token")
             bt[i, :len(seq.blocks)] = seq.blocks
             if n == 1:
                 ids[at], pos[at], slots[at] = seq.tokens[s0], s0, seq.blocks[s0 // KV_BLOCK] * KV_BLOCK + s0 % KV_BLOCK

@@ -51,6 +51,18 @@ def test_block_manager_prefix_sharing_and_lru():
         bm.allocate(1)
 
 
+@pytest.mark.parametrize("computed,n", [(KV, 1), (KV - 1, 2), (10, 2 * KV), (0, KV + 1)])
+def test_a_batch_of_tokens_past_the_blocks_of_their_sequence_is_refused(model, computed, n):
+    eng = LLMEngine(model, EngineOptions(max_ctx=512, max_seqs=2))
+    s = Sequence(0, [], SamplingParams(), tokens=list(range(computed + n)))
+    s.blocks, s.n_computed = [3], computed                         # one block: its tokens must not be sent to the null block of the table's other entries
+    with pytest.raises(IndexError):
+        eng._build_batch([(s, n)], [n - 1])
+    s.blocks = [3, 5, 4]
+    host, _ = eng._build_batch([(s, n)], [n - 1])
+    assert host["slot_map"].tolist() == [s.blocks[p // KV] * KV + p % KV for p in range(computed, computed + n)]
+
+
 def test_continuous_batching_matches_sequential(model):
     V = model.cfg.vocab
     prompts = [[(i * 7 + j) % V for i in range(n)] for j, n in enumerate((5, 140, 33, 260))]
