@@ -538,14 +538,17 @@ def _pick_bn(M: int, N: int, wide: bool = False) -> int:
     return 256 if wide and 1.71 * waves(256) < waves(128) else 128
 
 
-def _takes_pair(M: int, N: int) -> bool:
+def _takes_pair(M: int, N: int, K: int = 4096) -> bool:
     """Whether a bf16 product of more than 128 rows runs on pairs of SMs (``csrc/cuda/gemm_pair.cu``, 256 x 256 tiles, the same values bit for bit): where its
     waves are shorter.  In units of a wave of 128-row tiles of 64 or 128 columns (which take about as long, 26 us at K = 4096) a wave of 256 columns
     takes 1.95 and one of pair tiles 1.45 (39 us).  Both sides measured, us, other -> pair: 4096 x 28672 x 4096 742 -> 675, 4096 x 5120 x 2880 138 -> 92, 512 x
-    6144 x 4096 56 -> 46; it stays away from 256 x 4096 x 4096 (32 -> 44, one wave of 64 columns) and 300 x 28672 x 4096 (106 -> 111)."""
+    6144 x 4096 56 -> 46; it stays away from 256 x 4096 x 4096 (32 -> 44, one wave of 64 columns) and 300 x 28672 x 4096 (106 -> 111).  Against two waves of 64
+    columns its start weighs more than what a short K saves: 640 x 2048 x 512 11.3 -> 13.3, 200 x 8192 x 1536 18.4 -> 19.5, 400 x 2048 x 2048 even."""
     if M <= 128:
         return False
     sms, bn = sm_count(), _pick_bn(M, N, wide=True)
+    if bn == 64 and K < 2048:
+        return False
     waves = -(-(-(-M // 128) * -(-N // bn)) // sms)
     return 1.45 * -(-(-(-M // 256) * -(-N // 256)) // (sms // 2)) < waves * (1.95 if bn == 256 else 1.0)
 
@@ -582,24 +585,64 @@ def _few_rows_take_gemm(M: int, w: QuantWeight, act: int) -> bool:
 GEMM_ROWS_Q8_MAX = 40     # dense Q8 layers take the weight-streaming kernel (csrc/cuda/gemm_rows.cu) up to this many rows
 
 
-def _takes_rows(x, w: QuantWeight, act: int, row_scale) -> bool:
-    """Whether a dense layer of a few rows takes the weight-streaming kernel.  Measured with cold caches (us, GEMV or tcgen05 kernel -> this one):
-    two rows stay with the GEMV (6144 x 4096: bf16 21.4 -> 22.6, Q8 19.3 -> 23.5) except for gated bf16 and Q8 (28672 x 4096: 104 -> 58, 56 -> 42), which it reads
-    once per row; three rows 27.5 -> 23.4 and 25.4 -> 23.4, eight 55 -> 23 and 48 -> 24, forty 38 -> 29 and 64 -> 36.  Above: bf16 48 rows 38 -> 30, 64 rows
-    38 -> 34 but 30 -> 33 for 5120 x 2880; matrices of several full waves (from 100 M elements) are already near the memory rate in the tcgen05
-    kernel: 28672 x 4096 33 rows 71 -> 63, 48 rows 71 -> 70, 32768 x 4096 24 rows 68 -> 66, 33 rows 68.6 -> 69.7.  Q8 40 rows 64 -> 36 and 97 -> 69; 48 rows would
-    still gain (64 -> 32), but between there and DEQUANT_ONCE_MIN_M the values are those of the in-kernel decode that :func:`gemm` gives, bit for bit."""
-    M, big = x.shape[0], w.N * w.K >= 100 << 20
-    if w.fmt == WFormat.BF16:
-        most = 32 if big else 48
-    elif w.fmt == WFormat.Q8:
-        most = GEMM_ROWS_Q8_MAX
+def _rows_range(fmt, M: int, N: int, K: int, gated: bool) -> tuple:
+    """(fewest, most) rows of a dense layer that takes the weight-streaming kernel; below run the GEMVs, above the tcgen05 kernel.  us a call in a graph of calls
+    with cold caches, other kernel -> this one.
+
+    Fewest.  Its launch, merge and pipeline cost more than a GEMV's, which reads a matrix once up to 8 rows (gated: once per row) at a time that grows with the
+    rows.  bf16: 3 rows of 1536 x 4096 8.7 -> 11.1, 3072 x 2048 7.8 -> 10.6, 4096 x 2048 8.9 -> 8.9, 4096 x 4096 15.0 -> 14.0; 5 rows of 2048 x 2048 8.2 -> 8.4, 4096
+    x 1024 8.9 -> 7.5; 8 rows of 512 x 2048 6.0 -> 6.7, 2048 x 2048 8.4 -> 8.1, 6144 x 4096 48 -> 16; gated, 2 rows of 192 x 512 5.8 -> 5.1, 28672 x 4096 92 -> 43.
+    Q8: 3 rows of 4096 x 2048 9.1 -> 9.9, 1024 x 4096 11.3 -> 10.1; gated, 2 rows of 8192 x 4096 15.2 -> 16.2, 28672 x 4096 42 -> 35, 3 rows of 4096 x 2048 9.2 -> 9.9, 4 rows
+    2048 x 2048 7.8 -> 8.4, 4096 x 2048 11.1 -> 9.9, 5 rows 2048 x 512 7.8 -> 6.0, 192 x 512 5.3 -> 6.0.
+
+    Most.  The tcgen05 kernel's time is a chain over K per wave of tiles of 32 columns (one wave up to 32 x 148 columns), whatever the rows; this one grows with
+    the rows.  One wave, bf16: 512 columns of K 2048 24 rows 11.6 -> 10.2, 32 rows 11.4 -> 11.8; 4096 x 1024 24 rows 11.1 -> 9.9, 28 rows 10.9 -> 14.8; 3072 x 2048 31
+    rows 16.2 -> 15.5, 32 rows 12.1 -> 15.2; 2048 x 512 16 rows 7.2 -> 6.7, 20 rows 7.0 -> 7.8; 2880 x 4096 32 rows 18.9 -> 16.9, 33 rows 18.8 -> 20.3; 1024 x 4096 48
+    rows 18.4 -> 17.2; 2048 x 8192 48 rows 32 -> 22.  More waves: 6144 x 4096 48 rows 33 -> 22, 12288 x 2048 32 rows 21.0 -> 20.5, 40 rows 21.5 -> 23.2, 8192 x 1024 40 rows
+    16.4 -> 12.8, 6144 x 1024 40 rows 14.2 -> 14.8, 48 rows 14.0 -> 16.0, 8192 x 512 32 rows 10.8 -> 10.2, 40 rows 10.6 -> 11.6; matrices of several full waves (from 100 M elements) are near the memory rate there too: 28672 x 4096 33 rows 58.4 -> 58.7.  Gated layers
+    (one wave): 192 x 512 24 rows 8.2 -> 7.4, 32 rows 8.4 -> 9.4; 4096 x 2048 40 rows 14.2 -> 13.8, 48 rows 14.2 -> 16.0; 2048 x 2048 32 rows 13.7 -> 16.0 (runs of three steps cut the 32 of a
+    tile unevenly), 40 rows 13.7 -> 12.8.  Q8 40 rows 60 -> 22 for 6144 x 4096, but 2048 x 512 24 rows 8.7 -> 8.0, 32 rows 8.5 -> 9.9; 48 rows would still gain (60 -> 24), but
+    between there and DEQUANT_ONCE_MIN_M the values are those of the in-kernel decode that :func:`gemm` gives, bit for bit."""
+    size, one_wave = N * K, N <= 32 * sm_count()
+    if fmt == WFormat.Q8:
+        if gated:
+            fewest = 2 if size > 40 << 20 else 3 if size > 8 << 20 else 4 if size > 4 << 20 else 5 if size > 1 << 18 else 7
+        else:
+            fewest = 4 if K <= 2048 and size <= 8 << 20 else 3
+        return fewest, 24 if K < 1024 else GEMM_ROWS_Q8_MAX
+    fewest = 2
+    if not gated:
+        fewest = 3 if size > 7 << 20 or N > 6144 else 5 if size > (9 << 19 if N <= 2048 else 5 << 19) else 7 if size > 5 << 19 else 9
+    if size >= 100 << 20:
+        most = 32
+    elif gated:
+        most = 48 if not one_wave or K >= 2880 else 24 if K <= 1024 or (N <= 2048 and 24 < M <= 32) else 40
+    elif not one_wave:
+        most = 32 if K <= 512 or (K <= 2048 and N > 64 * sm_count()) else 40 if K <= 1024 else 48
+    elif K > 4096 or (K >= 2880 and N <= 1024):
+        most = 48
+    elif K >= 2880:
+        most = 32
+    elif K >= 1536:
+        most = (31 if K >= 2048 else 32) if N > 2048 else 40 if N <= 128 and K >= 2048 else 24
     else:
+        most = 24 if K >= 1024 else 16
+    return fewest, most
+
+
+def _takes_rows(x, w: QuantWeight, act: int, row_scale) -> bool:
+    """Whether a dense layer of a few rows takes the weight-streaming kernel (:func:`_rows_range`; layers with a row scale from one row on, since the GEMVs
+    have none).  Rows too long for the GEMV's shared memory, or too much weight for its arithmetic (:func:`_few_rows_take_gemm`), are no reason to go
+    back to it."""
+    M = x.shape[0]
+    if w.fmt not in (WFormat.BF16, WFormat.Q8) or M > 48 or w.K % 8 or x.data_ptr() % 16 or w.p0.data_ptr() % 16:
         return False
-    least = 2 if act_gated(act) else 3
+    fewest, most = _rows_range(w.fmt, M, w.N, w.K, act_gated(act))
     if row_scale is not None:
-        least = 1                        # (the GEMVs have no row scale)
-    return least <= M <= most and w.K % 8 == 0 and x.data_ptr() % 16 == 0 and w.p0.data_ptr() % 16 == 0
+        fewest = 1
+    elif M < fewest and _few_rows_take_gemm(M, w, act):
+        fewest = 3
+    return fewest <= M <= most
 
 
 def expert_chunk(w: QuantWeight, rows_per_expert: float) -> int:
@@ -660,7 +703,7 @@ def linear(x, w: QuantWeight, bias=None, act=ACT_NONE, act_alpha=1.702, act_limi
             _check(lib.mx_dequant_bf16(fmt, p0, p1, p2, p3, C.c_longlong(w.N), w.K, _p(wb), _stream()), "dequant_bf16")
             _count()
             fmt, p0, p1, p2, p3 = int(WFormat.BF16), _p(wb), _vp(0), _vp(0), _vp(0)
-        if fmt == int(WFormat.BF16) and _takes_pair(M, w.N):
+        if fmt == int(WFormat.BF16) and _takes_pair(M, w.N, w.K):
             _check(lib.mx_gemm_pair(_p(xa), p0, _p(out), out.stride(0), int(out_f32), _p(bias), _p(row_scale), act, C.c_float(act_alpha), C.c_float(act_limit),
                                     M, w.N, w.K, _stream()), "gemm_pair")
         else:
