@@ -8,7 +8,7 @@
 //   * the weights are the M side of mma.m16n8k16 and the activation rows its N side: 8 rows per column group, no padding to 128;
 //   * one warp issues TMA boxes of 128 weight rows x 128 bytes (and the activation rows' matching columns) into a ring of NST
 //     stages; four warps own 32 weight rows each and never wait for each other;
-//   * int8 codes go from the swizzled tile through ldmatrix to registers and are widened to bf16 exactly (three instructions per pair); each
+//   * int8 codes go from the swizzled tile through ldmatrix to registers and are widened to bf16 exactly (four instructions per pair); each
 //     32-element block is summed on its own and scaled in fp32, so the weights are not rounded to bf16;
 //   * up to 8 rows of bf16, where the GEMVs of fp32 additions are the alternative: the tensor cores cut a running sum off where an addition rounds (4096
 //     x 4096, error against 64 bits 4.0e-7 that way, 0.87e-7 in the GEMV), so every instruction's 16 products are summed on their own, and the
@@ -19,7 +19,8 @@
 //
 // Measured (B200, cold caches, before -> now): bf16 40 x 6144 x 4096 33.6 -> 20.8 us, 16 x 28672 x 4096 71 -> 58 (a bare stream of those weights through
 // the same ring takes 53: what is left is the launch, the partials of cut tiles and the epilogue); Q8 16 x 28672 x 4096 100 -> 47, 512 experts of
-// Q8 1024 x 2048 and 2048 x 512 with 19.5 rows each 1174 -> 888 (there the widening of the codes bounds it: ALU pipe 58 % active).
+// Q8 1024 x 2048 and 2048 x 512 with 19.5 rows each 1181 -> 823 (there the widening of the codes bounds it; looking up every tile of a run, instead of
+// stepping from one to the next, took 56 us of it).
 //
 // Bank conflicts: weight and activation tiles have the 128-byte TMA swizzle, ldmatrix rows differ in their low three bits.  With int8 codes a lane
 // holds four consecutive k, so its activations are 8-byte loads; column g of a group is row 2 (g & 3) + g / 4 of it, which spreads the
@@ -49,7 +50,7 @@ struct GemmRowsParams {
   const int* tile_expert;                // grouped: expert and live rows of every 128-row tile of A, number of tiles
   const int* tile_valid;
   const int* num_tiles;
-  int max_tiles;
+  int max_tiles, max_valid;              // tiles of more live rows than max_valid are left out
   float* part;                           // [grid][2][warp][2 NT][32] float4
   int* tickets;                          // [grid][warp]
   int* status;
@@ -130,6 +131,7 @@ __global__ void __launch_bounds__(GemmRowsShape<Q8, NT>::WARPS * 32 + 32, 2) gem
   __shared__ __align__(8) uint64_t s_bar[2 * NST + 2 * GR_WARPS];
   __shared__ int s_abort;
   __shared__ int s_pre[GR_MAX_ENTRIES + 1];                  // grouped: groups of rows before tile i
+  __shared__ uint8_t s_valid[GR_MAX_ENTRIES];                // and its live rows
   __shared__ int s_sum[S::WARPS + 1];
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -158,7 +160,9 @@ __global__ void __launch_bounds__(GemmRowsShape<Q8, NT>::WARPS * 32 + 32, 2) gem
     int run = 0;
     for (int i0 = 0; i0 < live_tiles; i0 += S::WARPS * 32 + 32) {
       const int i = i0 + tid;
-      const int valid = i < live_tiles ? p.tile_valid[i] : 0;
+      int valid = i < live_tiles ? p.tile_valid[i] : 0;
+      if (valid > p.max_valid) valid = 0;
+      if (i < live_tiles) s_valid[i] = (uint8_t)valid;
       int incl = valid / p.chunk * cost(p.chunk) + (valid % p.chunk ? cost(valid % p.chunk) : 0);
       const int own = incl;
 #pragma unroll
@@ -187,36 +191,46 @@ __global__ void __launch_bounds__(GemmRowsShape<Q8, NT>::WARPS * 32 + 32, 2) gem
 
   // A run is walked step by step: position `at` (in units of cost) of the step's start.  A step belongs to the CTA in whose run it starts.
   struct Place { int e, row0, rows, nt, cost, start, k; };   // start: position of the tile's first step; k: step
-  auto place = [&](int pos) {                                // the first step that starts at or after pos
+  auto advance = [&](Place& r) {                             // the next tile's first step (past the list: its start is `total`)
+    r.start += p.k_steps * r.cost;
+    r.k = 0;
+    if (++r.nt < p.n_tiles || !grouped) return;
+    r.nt = 0;
+    int i = r.row0 >> 7;
+    if ((r.row0 & 127) + p.chunk < s_valid[i]) {
+      r.row0 += p.chunk;
+    } else {
+      do ++i; while (i < live_tiles && !s_valid[i]);
+      r.row0 = i * 128;
+      r.e = i < live_tiles ? p.tile_expert[i] : 0;
+    }
+    r.rows = i < live_tiles ? min(p.chunk, s_valid[i] - (r.row0 & 127)) : 1;
+    r.cost = cost(r.rows);
+  };
+  auto place = [&](int pos) {                                // the first step that starts at or after pos (< total)
     Place r;
     r.e = 0; r.row0 = 0; r.rows = p.M; r.cost = 1;
     int base_pos = 0;
     if (grouped) {
       const int g = pos / steps_of;                          // cost units before: the tile of A with s_pre <= g
-      int lo = 0, hi = live_tiles - 1;                       // (a live tile has at least one row, so s_pre grows)
+      int lo = 0, hi = live_tiles - 1;                       // (the last one: tiles left out start where the next tile does)
       while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
         if (s_pre[mid] <= g) lo = mid; else hi = mid - 1;
       }
-      const int full = cost(p.chunk), valid = p.tile_valid[lo];
-      int c = (pos - s_pre[lo] * steps_of) / (full * steps_of);
-      r.rows = min(p.chunk, valid - c * p.chunk);
+      const int full = cost(p.chunk), c = (pos - s_pre[lo] * steps_of) / (full * steps_of);
+      r.rows = min(p.chunk, s_valid[lo] - c * p.chunk);
       r.cost = cost(r.rows);
-      base_pos = s_pre[lo] * steps_of + c * full * steps_of;
-      int i = (pos - base_pos + r.cost - 1) / r.cost;
-      if (i == steps_of) {                                   // between the last step of a group and the next group
-        base_pos += r.cost * steps_of;
-        if ((c + 1) * p.chunk < valid) ++c; else { ++lo; c = 0; }
-        r.rows = lo < live_tiles ? min(p.chunk, p.tile_valid[lo] - c * p.chunk) : 1;
-        r.cost = cost(r.rows);
-      }
-      r.e = lo < live_tiles ? p.tile_expert[lo] : 0;
+      r.e = p.tile_expert[lo];
       r.row0 = lo * 128 + c * p.chunk;
+      base_pos = s_pre[lo] * steps_of + c * full * steps_of;
     }
-    const int i = (max(pos - base_pos, 0) + r.cost - 1) / r.cost;
+    const int i = (pos - base_pos + r.cost - 1) / r.cost;
     r.nt = i / p.k_steps;
     r.k = i - r.nt * p.k_steps;
+    if (r.nt == p.n_tiles) { --r.nt; r.k = p.k_steps; }      // between the last step of a group and the next group
     r.start = base_pos + r.nt * p.k_steps * r.cost;
+    if (r.k == p.k_steps) advance(r);
     return r;
   };
 
@@ -237,9 +251,8 @@ __global__ void __launch_bounds__(GemmRowsShape<Q8, NT>::WARPS * 32 + 32, 2) gem
         if (Q8) tma_load_2d(st + S::X_BOX, &tm_x, bar_full + 8 * s, at.k * S::KS + 64, at.row0);
       };
       auto next = [&](Place& at) {                           // (false: past the run)
-        const int pos = at.start + (at.k + 1) * at.cost;
-        if (pos >= my1) return false;
-        if (++at.k == p.k_steps) at = place(pos);
+        if (at.start + (at.k + 1) * at.cost >= my1) return false;
+        if (++at.k == p.k_steps) advance(at);
         return true;
       };
       Place at = place(my0);
@@ -280,10 +293,11 @@ __global__ void __launch_bounds__(GemmRowsShape<Q8, NT>::WARPS * 32 + 32, 2) gem
     }
     uint32_t s = 0, ph = 0;
     bool ok = true;
-    for (int u = my0; u < my1 && ok;) {
-      const Place at = place(u);
+    Place at;
+    at.start = total; at.k = at.cost = 0;
+    if (my0 < my1) at = place(my0);
+    for (; ok && at.start + at.k * at.cost < my1; advance(at)) {
       const int first = at.k, n = min((my1 - at.start + at.cost - 1) / at.cost, p.k_steps) - first;      // steps that start before the run's end
-      if (n <= 0) break;
       const int nt_live = (at.rows + 7) / 8;
       float acc[2][NT][4];
 #pragma unroll
@@ -399,7 +413,6 @@ __global__ void __launch_bounds__(GemmRowsShape<Q8, NT>::WARPS * 32 + 32, 2) gem
           __syncwarp();
           if (lane == 0) mbar_arrive(full);
           xch_ph ^= 1;
-          u = at.start + (first + n) * at.cost;
           continue;
         }
         if (!(ok = mbar_wait(full, xch_ph, p.status, ERR_MBAR_TIMEOUT_MMA, abort_flag))) break;
@@ -435,7 +448,6 @@ __global__ void __launch_bounds__(GemmRowsShape<Q8, NT>::WARPS * 32 + 32, 2) gem
           if (prev == c1 - c0) p.tickets[c0 * GR_WARPS + wr] = 0;
         }
         prev = __shfl_sync(0xffffffffu, prev, 0);
-        u = at.start + (first + n) * at.cost;
         if (prev != c1 - c0) continue;
         __threadfence();
 #pragma unroll
@@ -472,8 +484,6 @@ __global__ void __launch_bounds__(GemmRowsShape<Q8, NT>::WARPS * 32 + 32, 2) gem
                 }
           }
         }
-      } else {
-        u = at.start + p.k_steps * at.cost;
       }
 
       // ---- epilogue: a lane holds weight rows g, g + 8 (and 16 further: the up rows of a gated pair) of columns 2 t4, 2 t4 + 1
@@ -565,11 +575,11 @@ MX_HOST_API int mx_gemm_rows_run(int total, int grid, int steps_nt, int cost) { 
 
 // C[M, N (/2 when gated)] = A[M,K] W[(E,) N, K]^T (+ bias, activation, row scale).  wfmt bf16 or Q8 (w1: scales, rows padded to 16 bytes).  Dense: M <= 64 and
 // tile_expert null.  Grouped: A is packed in 128-row tiles (tile_expert, tile_valid, num_tiles on the device, at most max_tiles of them: mx_gemm_rows_takes), taken in
-// groups of `chunk` rows; rows past a tile's live ones are not written.  tickets: see host_util.h.  out_kind 0 bf16, 1 fp32, 2 fp16.
+// groups of `chunk` rows; rows past a tile's live ones, and tiles of more than max_valid of them, are not written.  tickets: see host_util.h.  out_kind 0 bf16, 1 fp32, 2 fp16.
 MX_HOST_API int mx_gemm_rows(const void* a, int wfmt, const void* w0, const void* w1, int n_experts, void* c, int ldc, int out_kind, const float* bias,
                              const float* row_scale, int act, float act_alpha, float act_limit, int M, int N, int K, const int* tile_expert,
-                             const int* tile_valid, const int* num_tiles, int max_tiles, int chunk, float* scratch, int* tickets,
-                             cudaStream_t st) {
+                             const int* tile_valid, const int* num_tiles, int max_tiles, int max_valid, int chunk, float* scratch,
+                             int* tickets, cudaStream_t st) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   const bool q8 = wfmt == WF_Q8;
   if ((!q8 && wfmt != WF_BF16) || K % 8 || (q8 && K % 32)) return -101;
@@ -580,7 +590,7 @@ MX_HOST_API int mx_gemm_rows(const void* a, int wfmt, const void* w0, const void
   GemmRowsParams p;
   p.M = M; p.N = N; p.K = K; p.n_tiles = (N + GR_ROWS - 1) / GR_ROWS; p.k_steps = (K + ks - 1) / ks; p.chunk = chunk;
   p.C = c; p.ldc = ldc; p.out_f32 = out_kind; p.bias = bias; p.row_scale = row_scale; p.act = act; p.act_alpha = act_alpha; p.act_limit = act_limit;
-  p.tile_expert = tile_expert; p.tile_valid = tile_valid; p.num_tiles = num_tiles; p.max_tiles = max_tiles; p.part = scratch; p.status = status_word();
+  p.tile_expert = tile_expert; p.tile_valid = tile_valid; p.num_tiles = num_tiles; p.max_tiles = max_tiles; p.max_valid = max_valid; p.part = scratch; p.status = status_word();
   p.tickets = tickets;
   CUtensorMap tw, tx, td;
   {

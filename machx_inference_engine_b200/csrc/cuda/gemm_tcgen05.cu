@@ -59,7 +59,10 @@ struct GemmParams {
   const __nv_bfloat16* gate;
   int gate_ld;
   const int* a_pages;           // paged activations: m-tile i reads page a_pages[i] (BM rows each), null = row i * BM
+  const int* tile_valid;        // grouped Q8, 128 columns: only m-tiles of more than `min_valid` live rows are multiplied; null = all
+  int min_valid;
 };
+constexpr int kMaxFiltered = 1024;               // m-tiles of a launch with tile_valid
 
 constexpr int kRawDepth = 10;   // k-iterations of packed weight bytes kept in flight per producer thread
 
@@ -129,6 +132,40 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
+  constexpr bool kFilter = FMT == WF_Q8 && BN == 128;
+  if (kFilter && p.tile_valid) pdl_prologue();   // (launched while the weight-streaming kernel drains)
+  int m_tiles = p.num_m_tiles_dev ? min(*p.num_m_tiles_dev, p.num_m_tiles) : p.num_m_tiles;
+  // m-tiles taken, in their order: the others belong to the weight-streaming kernel (gemm_rows.cu).  A list, so that the CTAs share what is left evenly.
+  __shared__ uint16_t s_taken[kFilter ? kMaxFiltered : 1];
+  if constexpr (kFilter) {
+    static_assert(L::TOTAL + sizeof(s_taken) + 256 <= 232448, "shared memory plan exceeds 227 KB");
+    if (p.tile_valid) {
+      constexpr int WARPS = 448 / 32, ROUNDS = (kMaxFiltered + 447) / 448;
+      __shared__ uint32_t s_mask[ROUNDS * WARPS];
+#pragma unroll
+      for (int r = 0; r < ROUNDS; ++r) {
+        const int i = r * 448 + threadIdx.x;
+        const uint32_t mask = __ballot_sync(0xffffffffu, i < m_tiles && p.tile_valid[i] > p.min_valid);
+        if (lane == 0) s_mask[r * WARPS + warp] = mask;
+      }
+      __syncthreads();
+      int n = 0;
+#pragma unroll
+      for (int g = 0; g < ROUNDS * WARPS; ++g) {
+        const uint32_t mask = s_mask[g];
+        if (g % WARPS == warp && (mask >> lane & 1)) s_taken[n + __popc(mask & ((1u << lane) - 1))] = (uint16_t)(g * 32 + lane);
+        n += __popc(mask);
+      }
+      m_tiles = n;
+      if (n == 0) return;                        // (the same in every CTA, before any barrier or tensor memory)
+      __syncthreads();
+    }
+  }
+  auto taken = [&](int mt) {
+    if constexpr (kFilter) return p.tile_valid ? (int)s_taken[mt] : mt;
+    else return mt;
+  };
+
   if (threadIdx.x == 0) {
     for (int s = 0; s < SA; ++s) {
       mbar_init(bar_full + 8 * s, 1);
@@ -154,7 +191,6 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
 
-  const int m_tiles = p.num_m_tiles_dev ? min(*p.num_m_tiles_dev, p.num_m_tiles) : p.num_m_tiles;
   const int total_tiles = m_tiles * p.num_n_tiles;
   const int next_seq = p.peer.world ? *p.peer.seq + 1 : 0;
   const int k_iters = (p.K + BK - 1) / BK;
@@ -170,6 +206,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
         int mt, nt;
         tile_coords(t, m_tiles, p.num_n_tiles, p.group_m, mt, nt, p.m_rot);
+        mt = taken(mt);
         const int e = p.batch_tiles ? mt / p.batch_tiles : (p.tile_expert ? p.tile_expert[mt] : 0);
         const int a_row = (p.batch_tiles ? mt - e * p.batch_tiles : (p.a_pages ? p.a_pages[mt] : mt)) * BM;
         if (p.a_flags) {
@@ -241,6 +278,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
     for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x, ++tile_n) {
       int mt, nt;
       tile_coords(t, m_tiles, p.num_n_tiles, p.group_m, mt, nt, p.m_rot);
+      mt = taken(mt);
       const int e = p.batch_tiles ? mt / p.batch_tiles : (p.tile_expert ? p.tile_expert[mt] : 0);
       const uint32_t acc = tile_n & 1, acc_ph = (tile_n >> 1) & 1;
       if (!(ok = mbar_wait(bar_tfull + 8 * acc, acc_ph, p.status, ERR_MBAR_TIMEOUT_EPILOGUE, abort_flag))) break;
@@ -417,6 +455,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ 
       if (pt < total_tiles && live) {
         int pmt, pnt;
         tile_coords(pt, m_tiles, p.num_n_tiles, p.group_m, pmt, pnt, p.m_rot);
+        pmt = taken(pmt);
         const int n = pnt * BN + rl;
         if (n < p.N) {
           const int pe = p.tile_expert ? p.tile_expert[pmt] : 0;
@@ -503,7 +542,8 @@ static int launch(const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams
   const int tiles = p.num_m_tiles * p.num_n_tiles;
   const int grid = tiles < sm_count() ? tiles : sm_count();
   if (grid <= 0) return 0;
-  kern<<<grid, FMT == WF_BF16 ? 192 : 448, L::TOTAL, st>>>(ta, tb, p);
+  if (p.tile_valid) launch_pdl(kern, dim3(grid), dim3(448), L::TOTAL, st, ta, tb, p);
+  else kern<<<grid, FMT == WF_BF16 ? 192 : 448, L::TOTAL, st>>>(ta, tb, p);
   return (int)cudaGetLastError();
 }
 
@@ -533,6 +573,7 @@ static int dispatch_fmt(int fmt, const CUtensorMap& ta, const CUtensorMap& tb, c
 struct GatherIn { const int* flags; const int* seq; int rows_per_src, world, m_rot; };
 // Activations that are not one dense matrix: per head (heads > 0: row t of head h at a + t * lda + h * a_head, output at c + h * c_head) or pages
 // of 128 rows (pages: page number per m-tile, a_rows rows in all, lda elements apart).
+struct FilterIn { const int* tile_valid; int min_valid; };
 struct StridedIn {
   int heads = 0, lda = 0, gate_ld = 0;
   long long a_head = 0, c_head = 0, a_rows = 0;
@@ -542,7 +583,7 @@ struct StridedIn {
 static int gemm_impl(const void* a, int wfmt, const void* w0, const void* w1, const void* w2, const void* w3, int n_experts,
                      void* c, int ldc, int out_f32, const float* bias, const float* row_scale, int act, float act_alpha,
                      float act_limit, int M, int N, int K, const int* tile_expert, const int* num_m_tiles_dev, int bn,
-                     const mx::PeerOut* peer, cudaStream_t stream, const GatherIn* gin = nullptr, const StridedIn* sin = nullptr);
+                     const mx::PeerOut* peer, cudaStream_t stream, const GatherIn* gin = nullptr, const StridedIn* sin = nullptr, const FilterIn* fin = nullptr);
 
 MX_HOST_API int mx_gemm(const void* a, int wfmt, const void* w0, const void* w1, const void* w2, const void* w3, int n_experts,
                         void* c, int ldc, int out_f32, const float* bias, const float* row_scale, int act, float act_alpha,
@@ -550,6 +591,16 @@ MX_HOST_API int mx_gemm(const void* a, int wfmt, const void* w0, const void* w1,
                         cudaStream_t stream) {
   return gemm_impl(a, wfmt, w0, w1, w2, w3, n_experts, c, ldc, out_f32, bias, row_scale, act, act_alpha, act_limit, M, N, K, tile_expert,
                    num_m_tiles_dev, bn, nullptr, stream);
+}
+
+// Grouped Q8 product over the m-tiles of more than `min_valid` live rows (tile_valid: live rows of every tile; at most 1024 tiles); the rows of the others
+// are not written.
+MX_HOST_API int mx_gemm_grouped_over(const void* a, const void* w0, const void* w1, int n_experts, void* c, int ldc, int out_kind, const float* bias, int act,
+                                     float act_alpha, float act_limit, int M, int N, int K, const int* tile_expert, const int* tile_valid,
+                                     const int* num_m_tiles_dev, int min_valid, cudaStream_t stream) {
+  const FilterIn f{tile_valid, min_valid};
+  return gemm_impl(a, mx::WF_Q8, w0, w1, nullptr, nullptr, n_experts, c, ldc, out_kind, bias, nullptr, act, act_alpha, act_limit, M, N, K, tile_expert,
+                   num_m_tiles_dev, 128, nullptr, stream, nullptr, nullptr, &f);
 }
 
 // all-gather -> GEMM: `a` is this rank's gather buffer [M,K]; rows [s * rows_per_src, (s + 1) * rows_per_src) are valid once
@@ -580,7 +631,7 @@ MX_HOST_API int mx_gemm_allreduce(const void* a, int wfmt, const void* w0, const
 static int gemm_impl(const void* a, int wfmt, const void* w0, const void* w1, const void* w2, const void* w3, int n_experts,
                      void* c, int ldc, int out_f32, const float* bias, const float* row_scale, int act, float act_alpha,
                      float act_limit, int M, int N, int K, const int* tile_expert, const int* num_m_tiles_dev, int bn,
-                     const mx::PeerOut* peer, cudaStream_t stream, const GatherIn* gin, const StridedIn* sin) {
+                     const mx::PeerOut* peer, cudaStream_t stream, const GatherIn* gin, const StridedIn* sin, const FilterIn* fin) {
   using namespace mx;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (K % 8) return -101;
@@ -606,6 +657,12 @@ static int gemm_impl(const void* a, int wfmt, const void* w0, const void* w1, co
     p.a_flags = gin->flags; p.a_seq = gin->seq; p.a_rows_per_src = gin->rows_per_src; p.a_world = gin->world;
     p.m_rot = gin->m_rot % p.num_m_tiles;
     p.group_m = 1;                                      // m-major walk: all n-tiles of a row chunk before the next chunk is needed
+  }
+
+  p.tile_valid = nullptr; p.min_valid = 0;
+  if (fin) {
+    if (wfmt != WF_Q8 || bn != 128 || !tile_expert || p.num_m_tiles > kMaxFiltered) return -107;
+    p.tile_valid = fin->tile_valid; p.min_valid = fin->min_valid;
   }
 
   p.batch_tiles = 0; p.c_batch = 0; p.gate = nullptr; p.gate_ld = 0; p.a_pages = nullptr;

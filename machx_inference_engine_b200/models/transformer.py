@@ -795,7 +795,7 @@ class MoEFFN:
             pk = ops.moe_pack(idx, self.E, self.e_lo, self.e_hi)
             xp = ops.moe_gather(h, pk)
             te = pk.tile_expert - self.e_lo if self.e_lo else pk.tile_expert
-            few = lambda w: dict(tile_valid=pk.tile_valid, chunk=ops.expert_chunk(w, T * self.K / self.E))
+            few = lambda w: dict(tile_valid=pk.tile_valid, chunk=ops.expert_chunk(w, T * self.K / self.E), tokens=T)
             a = ops.grouped_linear(xp, self.gate_up, te, pk.num_tiles, bias=self.gu_bias, act=self.act, **few(self.gate_up))
             y = ops.grouped_linear(a, self.down, te, pk.num_tiles, bias=self.down_bias, **few(self.down))
             if fuse_push:

@@ -647,22 +647,33 @@ def _takes_rows(x, w: QuantWeight, act: int, row_scale) -> bool:
 
 def expert_chunk(w: QuantWeight, rows_per_expert: float) -> int:
     """Rows per group with which a bank of experts takes the weight-streaming kernel, 0: the grouped tcgen05 kernel.  Q8 banks, gate / up and down, us at the mean
-    rows per expert (tcgen05 -> this kernel, groups of 8 / 16): 512 experts of 1024 x 2048: 0.6 rows 499 -> 206 / 210, 2.5 rows 957 -> 376 / 382,
-    10 rows 1082 -> 753 / 603, 19.5 rows 1174 -> 1248 / 888, 29 rows 1164 -> 1173; 128 of 1536 x 2048: 16 rows 433 -> 300, 32 rows 413 -> 468."""
+    rows per expert (tcgen05 -> this kernel): 512 experts of 1024 x 2048: 0.6 rows 587 -> 202, 2.5 rows 1085 -> 368, 10 rows 1182 -> 516, 19.5 rows 1181 -> 823, 23.4 rows
+    1179 -> 925; 128 of 1536 x 2048: 16 rows 426 -> 274; 64 of 2816 x 2048: 24 rows 405 -> 333, and 32 rows of 128 of 1536 x 2048 413 -> 468 (when a
+    tile still cost a search).  Groups of 8 and 16 cost the same up to 3 rows (376, 382), then 16 gain (10 rows 753, 603)."""
     if w.fmt != WFormat.Q8 or rows_per_expert > 24:
         return 0
     return 8 if rows_per_expert <= 3 else 16
 
 
-def _gemm_rows(x, w: QuantWeight, out, out_kind, bias, row_scale, act, act_alpha, act_limit, chunk, tiles=None):
-    """``tiles``: (tile_expert, tile_valid, num_tiles) of packed expert rows, taken in groups of ``chunk``.  The scratch (partials of cut tiles) is an ordinary
+def expert_rows_max(tokens: int) -> int:
+    """Live rows of a packed tile up to which it is streamed in groups, where an expert may have `tokens` rows: every group of 16 streams and widens the weights
+    again, which the tcgen05 kernel does once per tile of 128.  One tile there takes 25 us however few there are, so nothing is split off below 129
+    rows (128 tokens, all routed alike: 176 -> 165 us without).  Q8 banks of 512 experts of 1024 x 2048, 10 per token, gate / up and down, us (tcgen05 alone -> streamed alone ->
+    both, at 48 / 64 rows), scores of the experts spread by 0, 1 and 3 standard deviations: 256 tokens 1172 -> 440 -> 437 / 437, 588 -> 325 -> 340 / 350, 188 -> 215 -> 186 / 176;
+    1000 tokens 1181 -> 813 -> 825 / 823, 815 -> 800 -> 563 / 594, 325 -> 650 -> 335 / 318.  128 experts of 1536 x 2048, 256 tokens: 426 -> 268 -> 275 / 274, 347 -> 275 ->
+    267 / 280, spread 0.5 449 -> 276 -> 325 / 284."""
+    return 128 if tokens <= 128 else 64 if tokens <= 384 else 48
+
+
+def _gemm_rows(x, w: QuantWeight, out, out_kind, bias, row_scale, act, act_alpha, act_limit, chunk, tiles=None, max_valid=128):
+    """``tiles``: (tile_expert, tile_valid, num_tiles) of packed expert rows, taken in groups of ``chunk``, tiles of more than ``max_valid`` live rows left out.  The scratch (partials of cut tiles) is an ordinary
     allocation: stream-ordered, of the graph's own pool under capture."""
     lib = _lib.cuda()
     scratch = torch.empty(lib.mx_gemm_rows_scratch(chunk), dtype=torch.float32, device=x.device)
     tickets = _tickets(x.device)
     te, tv, nt = tiles if tiles is not None else (None, None, None)
     _check(lib.mx_gemm_rows(_p(x), int(w.fmt), _p(w.p0), _p(w.p1), w.E, _p(out), out.stride(0), out_kind, _p(bias), _p(row_scale), act, C.c_float(act_alpha),
-                            C.c_float(act_limit), x.shape[0], w.N, w.K, _p(te), _p(tv), _p(nt), 0 if te is None else te.numel(), int(chunk), _p(scratch),
+                            C.c_float(act_limit), x.shape[0], w.N, w.K, _p(te), _p(tv), _p(nt), 0 if te is None else te.numel(), int(max_valid), int(chunk), _p(scratch),
                             tickets[1], tickets[2]), "gemm_rows")
 
 
@@ -805,9 +816,10 @@ def gemm(x, w: QuantWeight, bias=None, act=ACT_NONE, act_alpha=1.702, act_limit=
 
 
 def grouped_linear(xp, w: QuantWeight, tile_expert, num_tiles, bias=None, act=ACT_NONE, act_alpha=1.702, act_limit=7.0, out_f32=False, bn=128,
-                   out_dtype=None, tile_valid=None, chunk=0):
+                   out_dtype=None, tile_valid=None, chunk=0, tokens=0):
     """``chunk`` > 0 (with ``tile_valid``, the live rows of every tile): the weight-streaming kernel over groups of that many rows, for experts of a few dozen
-    rows each; rows past a tile's live ones are then not written.  ``out_dtype`` (bf16 / fp16 / fp32) overrides ``out_f32``; fp16 feeds a following MXFP4 GEMM without a cast."""
+    rows each; rows past a tile's live ones are then not written.  ``tokens``: rows that one expert may have; tiles of more live rows than
+    :func:`expert_rows_max` says go to the tcgen05 kernel after all.  ``out_dtype`` (bf16 / fp16 / fp32) overrides ``out_f32``; fp16 feeds a following MXFP4 GEMM without a cast."""
     P = xp.shape[0]
     if xp.dtype == torch.float32:            # 32-bit models: every row in fp32 on the CUDA cores
         if w.fmt != WFormat.BF16 or bias is not None or out_dtype not in (None, torch.float32):
@@ -825,8 +837,13 @@ def grouped_linear(xp, w: QuantWeight, tile_expert, num_tiles, bias=None, act=AC
     fmt, p0, p1, p2, p3 = _planes(w)
     xp = _gemm_a(xp, w)
     if chunk and tile_valid is not None and w.fmt in (WFormat.BF16, WFormat.Q8) and _lib.cuda().mx_gemm_rows_takes(fmt, tile_expert.numel(), chunk, w.N, w.K):
-        _gemm_rows(xp, w, out, _out_kind(odt), bias, None, act, act_alpha, act_limit, chunk, tiles=(tile_expert, tile_valid, num_tiles))
+        limit = expert_rows_max(tokens) if w.fmt == WFormat.Q8 and bn == 128 else 128
+        _gemm_rows(xp, w, out, _out_kind(odt), bias, None, act, act_alpha, act_limit, chunk, tiles=(tile_expert, tile_valid, num_tiles), max_valid=limit)
         _count()
+        if limit < 128:
+            _check(_lib.cuda().mx_gemm_grouped_over(_p(xp), p0, p1, w.E, _p(out), n_out, _out_kind(odt), _p(bias), act, C.c_float(act_alpha), C.c_float(act_limit), P,
+                                                    w.N, w.K, _p(tile_expert), _p(tile_valid), _p(num_tiles), limit, _stream()), "grouped gemm")
+            _count()
         return out
     _check(_lib.cuda().mx_gemm(_p(xp), fmt, p0, p1, p2, p3, w.E, _p(out), n_out, _out_kind(odt), _p(bias), _vp(0), act, C.c_float(act_alpha),
                                C.c_float(act_limit), P, w.N, w.K, _p(tile_expert), _p(num_tiles), bn, _stream()), "grouped gemm")

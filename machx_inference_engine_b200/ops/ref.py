@@ -170,9 +170,9 @@ def hadamard128(x, pre=None, post=None, bias=None, out_f32=False, out=None):
 
 
 def grouped_linear(xp, w: QuantWeight, tile_expert, num_tiles, bias=None, act=ACT_NONE, act_alpha=1.702, act_limit=7.0, out_f32=False, bn=128,
-                   out_dtype=None, tile_valid=None, chunk=0):
-    """xp: packed rows [P,K]; tile t (rows 128t..128t+127) uses expert tile_expert[t] for t < num_tiles[0].  ``tile_valid`` (live rows of every tile) and
-    ``chunk`` choose a kernel on the GPU."""
+                   out_dtype=None, tile_valid=None, chunk=0, tokens=0):
+    """xp: packed rows [P,K]; tile t (rows 128t..128t+127) uses expert tile_expert[t] for t < num_tiles[0].  ``tile_valid`` (live rows of every tile),
+    ``chunk`` and ``tokens`` choose a kernel on the GPU."""
     W = _dense(w)
     P = xp.shape[0]
     n_out = w.N // 2 if act_gated(act) else w.N

@@ -128,3 +128,28 @@ def test_infinite_sums_stay_infinite():
     x[2, 4000] = float("nan")
     got = product(x, w, True)
     assert bool(torch.isposinf(got[:2]).all()) and bool(got[2].isnan().all()) and rel(got[3], x[3].double() @ values(w)[0].T) < 2.0 ** -21
+
+
+@pytest.mark.parametrize("T,E,k,chunk,limit", [(300, 16, 4, 16, 32), (40, 8, 3, 8, 32), (1000, 300, 2, 16, 1), (700, 5, 3, 16, 32), (260, 4, 2, 16, 127), (64, 40, 1, 8, 64)])
+def test_experts_of_many_rows_among_experts_of_few(T, E, k, chunk, limit, monkeypatch):
+    """Tiles of up to ``limit`` live rows in one kernel, the others in the other one: every pair's row is written once, whatever the order of the two kinds.  The
+    bf16 decode of the tcgen05 kernel rounds a weight by 2^-9 of itself: 2^-9 of the sum at most, and less than a third of it with independent terms."""
+    monkeypatch.setattr(K(), "expert_rows_max", lambda tokens: limit)
+    H, F, dev = 192, 320, "cuda:0"
+    gu, down = weight(WFormat.Q8, F, H, E, 1), weight(WFormat.Q8, 200, F // 2, E, 2)
+    x = torch.randn(T, H, device=dev).to(torch.bfloat16)
+    idx = (torch.randn(T, E, device=dev) + 3 * torch.randn(E, device=dev)).topk(k, dim=1).indices.int()
+    pk = K().moe_pack(idx, E)
+    xp = K().moe_gather(x, pk)
+    bias = torch.randn(E, F, device=dev)
+    kw = dict(tile_valid=pk.tile_valid, chunk=chunk, tokens=T, out_dtype=torch.float32)
+    a = K().grouped_linear(xp, gu, pk.tile_expert, pk.num_tiles, bias=bias, act=ops.ACT_SWIGLU, **kw)
+    at, e = pk.pair_to_packed.long(), idx.reshape(-1).long()
+    h = torch.einsum("pk,pnk->pn", x.double().repeat_interleave(k, 0), values(gu)[e]) + bias.double()[e]
+    gate, up = h.view(-1, F // 32, 2, 16).unbind(2)
+    assert rel(a[at], (torch.nn.functional.silu(gate) * up).reshape(T * k, F // 2)) < 2.0 ** -9
+    ab = a.to(torch.bfloat16)
+    y = K().grouped_linear(ab, down, pk.tile_expert, pk.num_tiles, **kw)
+    assert rel(y[at], torch.einsum("pk,pnk->pn", ab[at].double(), values(down)[e])) < 2.0 ** -9
+    assert torch.equal(y[at], K().grouped_linear(ab, down, pk.tile_expert, pk.num_tiles, **kw)[at])
+    K().check_status()
