@@ -101,11 +101,16 @@ def check_status():
         raise KernelError(f"kernel status {v}: {names.get(v, 'unknown')} ran out of its time limit")
 
 
+_gemv_path = 0
+
+
 def set_gemv_path(path) -> None:
     """Which decode GEMV kernel runs: "auto" (per case, the default), "register" (register-streamed kernels only) or
-    "stream" (the bulk-copy streaming kernel wherever it applies); booleans mean register / auto."""
-    code = {"auto": 0, "register": 1, "stream": 2, True: 1, False: 0}[path]
-    _lib.cuda().mx_gemv_set_path(code)
+    "stream" (the bulk-copy streaming kernel wherever it applies); booleans mean register / auto.  A path that is asked for is not
+    left to the weight-streaming kernel of few rows either."""
+    global _gemv_path
+    _gemv_path = {"auto": 0, "register": 1, "stream": 2, True: 1, False: 0}[path]
+    _lib.cuda().mx_gemv_set_path(_gemv_path)
 
 
 def set_gemv_bf16_wide(on: Optional[bool]) -> None:
@@ -635,7 +640,7 @@ def _takes_rows(x, w: QuantWeight, act: int, row_scale) -> bool:
     have none).  Rows too long for the GEMV's shared memory, or too much weight for its arithmetic (:func:`_few_rows_take_gemm`), are no reason to go
     back to it."""
     M = x.shape[0]
-    if w.fmt not in (WFormat.BF16, WFormat.Q8) or M > 48 or w.K % 8 or x.data_ptr() % 16 or w.p0.data_ptr() % 16:
+    if _gemv_path or w.fmt not in (WFormat.BF16, WFormat.Q8) or M > 48 or w.K % 8 or x.data_ptr() % 16 or w.p0.data_ptr() % 16:
         return False
     fewest, most = _rows_range(w.fmt, M, w.N, w.K, act_gated(act))
     if row_scale is not None:

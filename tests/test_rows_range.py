@@ -1,8 +1,10 @@
 """Which dense layers of a few rows take the weight-streaming kernel: sizes at which another kernel was measured to be faster stay with it."""
 import pytest
+import torch
 
+from machx_inference_engine_b200 import _build
 from machx_inference_engine_b200.ops import cuda as K
-from machx_inference_engine_b200.ops.weights import WFormat
+from machx_inference_engine_b200.ops.weights import QuantWeight, WFormat
 
 B, Q = WFormat.BF16, WFormat.Q8
 # format, rows, columns, depth, gated
@@ -29,3 +31,24 @@ def test_measured_sizes(case, here):
 def test_pairs_of_sms_stay_away_from_short_sums_in_few_tiles():
     for M, N, Kd, here in ((640, 2048, 512, False), (200, 8192, 1536, False), (640, 2048, 2048, True), (1024, 4096, 256, True), (4096, 28672, 4096, True), (256, 4096, 4096, False)):
         assert K._takes_pair(M, N, Kd) == here, (M, N, Kd)
+
+
+@pytest.mark.skipif(not _build.CUDA_LIB.exists() and _build._nvcc() is None, reason="no kernel library and no compiler")
+def test_a_gemv_path_that_is_asked_for_is_the_one_that_runs():
+    x, w = torch.zeros(8, 4096, dtype=torch.bfloat16), QuantWeight(B, 4096, 4096, 1, torch.zeros(1, 4096, 4096, dtype=torch.bfloat16))
+    assert K._takes_rows(x, w, 0, None)
+    try:
+        for path in ("stream", "register"):
+            K.set_gemv_path(path)
+            assert not K._takes_rows(x, w, 0, None), path
+    finally:
+        K.set_gemv_path("auto")
+    assert K._takes_rows(x, w, 0, None)
+
+
+@pytest.mark.parametrize("M", [3, 5, 6, 7])
+def test_long_rows_leave_the_gemv_only_while_it_serves_them_badly(M, monkeypatch):
+    x, w = torch.zeros(M, 12288, dtype=torch.bfloat16), QuantWeight(B, 64, 12288, 1, torch.zeros(1, 64, 12288, dtype=torch.bfloat16))
+    assert K._takes_rows(x, w, 0, None) == K._few_rows_take_gemm(M, w, 0) == (M > 5)
+    monkeypatch.setattr(K, "_few_rows_take_gemm", lambda *a: False)
+    assert not K._takes_rows(x, w, 0, None)
