@@ -296,8 +296,10 @@ __global__ void __launch_bounds__(DN_THREADS) deltanet_scan_kernel(ScanParams p)
 
 // ------------------------------------------------------------------ gated RMSNorm, z read through a row stride
 // Bound by memory: a warp takes four 16-byte vectors of every lane at once (four rows of up to 128 elements, two of up to 256), so that enough bytes are under
-// way.  VPR: vectors of a row per lane, 0: any width and alignment, one row per warp with scalar loads (4100 x 32 heads of 128, 134 MB: 49 us that way, 37 with
-// one vectorised row per warp, MEASURED with four).  The vector forms need 16-byte rows of x and w and 8-byte rows of z and y.
+// way.  VPR: vectors of a row per lane, 0: any width and alignment, one row per warp with scalar loads.  us a launch in a graph, VPR 0 -> 1: 4100 x 32 heads of 128 (134
+// MB) 46.7 -> 31.4, 500 x 32 8.2 -> 7.5, but 64 x 32 4.1 -> 4.4 and one token 3.4 -> 4.1: where a few warps hold all rows, one row each is the shorter chain
+// (up to GRN_FEW_ROWS; rows of 256 gain from the first, 16 of them 4.8 -> 3.8).  The vector forms need 16-byte rows of x and w and 8-byte rows of z and y.
+constexpr int GRN_FEW_ROWS = 4096;
 constexpr int GRN_VECS = 4;
 template <int VPR>
 __global__ void __launch_bounds__(128) gated_rmsnorm_ld_kernel(const float* __restrict__ x, const bf16* __restrict__ z, int z_ld,
@@ -404,8 +406,9 @@ MX_HOST_API int mx_gated_rmsnorm_ld(const float* x, const void* z, int z_ld, con
                                     cudaStream_t st) {
   if (T <= 0) return 0;
   const bool vec = hd % 4 == 0 && hd <= 256 && z_ld % 4 == 0 && (((uintptr_t)x | (uintptr_t)w) & 15) == 0 && (((uintptr_t)z | (uintptr_t)y) & 7) == 0;
-  auto kern = !vec ? gated_rmsnorm_ld_kernel<0> : hd <= 128 ? gated_rmsnorm_ld_kernel<1> : gated_rmsnorm_ld_kernel<2>;
-  const int per_cta = 4 * (!vec ? 1 : hd <= 128 ? GRN_VECS : GRN_VECS / 2);
+  const bool scalar = !vec || (hd <= 128 && (long long)T * n_h <= GRN_FEW_ROWS);
+  auto kern = scalar ? gated_rmsnorm_ld_kernel<0> : hd <= 128 ? gated_rmsnorm_ld_kernel<1> : gated_rmsnorm_ld_kernel<2>;
+  const int per_cta = 4 * (scalar ? 1 : hd <= 128 ? GRN_VECS : GRN_VECS / 2);
   launch_pdl(kern, dim3((T * n_h + per_cta - 1) / per_cta), dim3(128), 0, st, x, (const bf16*)z, z_ld, w, (bf16*)y, T, n_h, hd, eps);
   return (int)cudaGetLastError();
 }
