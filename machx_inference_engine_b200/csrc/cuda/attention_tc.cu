@@ -25,8 +25,9 @@
 // Bound: the exponentials (16 per SM and cycle: 122 us for 4096 causal tokens of 64 heads, against 85 us of tensor time with heads of 64).  One softmax
 // warp per scheduler cannot hide its own chain of TMEM read, maximum, exponentials and write, hence two CTAs per SM with half the tile each, P that never
 // passes shared memory, and packed fp32 arithmetic.
-// Measured (B200): 4096 causal tokens, 64 / 8 heads of 64: 418 -> 233 us (591 TFLOP/s, exponential unit 57 % active); six ragged prompts behind cached prefixes, 32 /
-// 8 heads of 128: 722 -> 694 us (868 TFLOP/s).  One CTA of 128-key tiles per SM, P through shared memory and the short query tiles first was the form before.
+// Measured (B200): 4096 causal tokens, 64 / 8 heads of 64: 418 -> 233 us (591 TFLOP/s); six ragged prompts behind cached prefixes, 32 / 8 heads of 128: 722 -> 652 us (924
+// TFLOP/s).  One CTA of 128-key tiles per SM, P through shared memory and the short query tiles first was the form before; it is still the faster one where an SM gets
+// no second CTA anyway (512 tokens behind 16000, 32 / 8 heads of 128: 191 -> 244 us) and by 5 to 10 % with heads of 256 there.
 // The per-head sink joins the denominator once, at the end.  Every wait is bounded.
 //
 // Reference parity: src/ops/attention.cpp:2456-2815 (fa2_tile_wide_impl<HD,Bc,REGDOT,SG,SINK> for HD 64..512 and its

@@ -606,7 +606,7 @@ def _rows_range(fmt, M: int, N: int, K: int, gated: bool) -> tuple:
     rows 18.4 -> 17.2; 2048 x 8192 48 rows 32 -> 22.  More waves: 6144 x 4096 48 rows 33 -> 22, 12288 x 2048 32 rows 21.0 -> 20.5, 40 rows 21.5 -> 23.2, 8192 x 1024 40 rows
     16.4 -> 12.8, 6144 x 1024 40 rows 14.2 -> 14.8, 48 rows 14.0 -> 16.0, 8192 x 512 32 rows 10.8 -> 10.2, 40 rows 10.6 -> 11.6; matrices of several full waves (from 100 M elements) are near the memory rate there too: 28672 x 4096 33 rows 58.4 -> 58.7.  Gated layers
     (one wave): 192 x 512 24 rows 8.2 -> 7.4, 32 rows 8.4 -> 9.4; 4096 x 2048 40 rows 14.2 -> 13.8, 48 rows 14.2 -> 16.0; 2048 x 2048 32 rows 13.7 -> 16.0 (runs of three steps cut the 32 of a
-    tile unevenly), 40 rows 13.7 -> 12.8.  Q8 40 rows 60 -> 22 for 6144 x 4096, but 2048 x 512 24 rows 8.7 -> 8.0, 32 rows 8.5 -> 9.9; 48 rows would still gain (60 -> 24), but
+    tile unevenly), 40 rows 13.7 -> 12.8.  Q8 40 rows 60 -> 22 for 6144 x 4096, but 2048 x 512 24 rows 8.7 -> 8.0, 32 rows 8.5 -> 9.9; 48 rows would still gain (64 -> 32 in single calls), but
     between there and DEQUANT_ONCE_MIN_M the values are those of the in-kernel decode that :func:`gemm` gives, bit for bit."""
     size, one_wave = N * K, N <= 32 * sm_count()
     if fmt == WFormat.Q8:
